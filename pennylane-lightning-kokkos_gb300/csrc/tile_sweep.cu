@@ -1,0 +1,270 @@
+// tile_sweep.cu — op lists and adjoint sweeps as tile programs.
+//
+// plk_apply_ops (StateVectorKokkos::applyOperation over a tape,
+// StateVectorKokkos.hpp:585-676) and plk_adjoint_jacobian
+// (AdjointDiffKokkos.hpp:404-478) compile their ops into passes over the state
+// (tile_program.hpp) and launch one kernel per pass (tile_kernels.cuh).  The
+// sweeps of several observables run in the same launches (gridDim.y), each on
+// its own copy of lambda.  Op lists with dense matrices keep the register
+// windows (windows.cu).
+#include <algorithm>
+#include <vector>
+
+#include "gate_ops.cuh"
+#include "tile_launch.cuh"
+
+namespace plk {
+
+bool window_path_enabled();
+int plan_generator(int gate, int nw, GatePlan &p);
+
+namespace tile {
+
+// jac[y][s] = sum over the slot's terms of coef * (the accumulator's sum over
+// CTAs); one warp per slot, CTAs in lane-strided order, fixed pattern
+__global__ void k_tile_jac(const double *__restrict__ part, int nblocks, int nacc_all, const int *__restrict__ first,
+                           const int *__restrict__ term_acc, const double *__restrict__ term_coef, int nslots,
+                           double *__restrict__ jac) {
+    const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (s >= nslots) return;
+    const double *p = part + (size_t)blockIdx.y * nacc_all * nblocks;
+    double t = 0.0;
+    for (int k = first[s]; k < first[s + 1]; k++) {
+        double a = 0.0;
+        for (int b = lane; b < nblocks; b += 32) a += p[(size_t)term_acc[k] * nblocks + b];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        t += term_coef[k] * a;
+    }
+    if (lane == 0) jac[(size_t)blockIdx.y * nslots + s] = t;
+}
+
+struct Shape {
+    int R, threads, ctas;
+};
+static Shape shape(int dtype, bool bwd) {
+    if (dtype == PLK_C64)
+        return bwd ? Shape{kRegsC64Bwd, kThreadsC64Bwd, kCtasC64Bwd} : Shape{kRegsC64Fwd, kThreadsC64Fwd, kCtasC64Fwd};
+    return bwd ? Shape{kRegsC128Bwd, kThreadsC128Bwd, kCtasC128Bwd}
+               : Shape{kRegsC128Fwd, kThreadsC128Fwd, kCtasC128Fwd};
+}
+
+static int tile_bits(int nq, int dtype, bool bwd) {
+    const Shape sh = shape(dtype, bwd);
+    int T = sh.R;
+    while ((1 << (T - sh.R)) < sh.threads) T++;
+    return std::min(T, nq);
+}
+
+static Options options(int nq, int dtype, bool bwd) {
+    Options o;
+    o.T = tile_bits(nq, dtype, bwd);
+    o.R = shape(dtype, bwd).R;
+    o.amp_bytes = dtype == PLK_C64 ? 8 : 16;
+    o.low = dtype == PLK_C64 ? 3 : 2; // 64-byte runs
+    o.max_blob = kMaxBlob;
+    return o;
+}
+
+static int check_program(const TileProgram &P, int amp_bytes) {
+    for (const TilePass &p : P.passes)
+        if (!check_pass(p, P.nq, amp_bytes, P.nacc)) PLK_FAIL(PLK_ERR_UNSUPPORTED, "internal: tile program check failed");
+    for (const JacTerm &t : P.jac)
+        if (t.acc < 0 || t.acc >= P.nacc) PLK_FAIL(PLK_ERR_UNSUPPORTED, "internal: tile program check failed");
+    return PLK_OK;
+}
+
+// Runs P on nsweep (lambda, H lambda) pairs on stream st.  Backward, the
+// Jacobian rows go to jac_host (row-major [nsweep][nslots]; synchronizes).
+static int run(const TileProgram &P, int dtype, int device, cudaStream_t st, const void *const *lam_src,
+               void *const *lam, void *const *hl, int nsweep, int nslots, double *jac_host) {
+    DeviceCtx *d = nullptr;
+    PLK_TRY(device_ctx(device, &d));
+    const bool c64 = dtype == PLK_C64;
+    PLK_TRY(check_program(P, c64 ? 8 : 16));
+    const Shape sh = shape(dtype, P.bwd);
+    const int threads = std::max(32, 1 << (P.T - P.R));
+    const int ntiles = 1 << (P.nq - P.T);
+    // one resident wave: CTAs walk their tiles
+    const int per_sm = std::min(sh.ctas * sh.threads / threads, 8);
+    // a tile of fewer threads than a warp is worked on by several lanes alike
+    const double share = (double)(1 << (P.T - P.R)) / threads;
+    const int gx = std::max(1, std::min(ntiles, d->sm_count * per_sm / nsweep));
+    // one device buffer: blobs, Jacobian terms, partial sums, Jacobian
+    auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    std::vector<size_t> at;
+    size_t up = 0;
+    for (const TilePass &p : P.passes) {
+        at.push_back(up);
+        up += al(p.blob.size());
+    }
+    const size_t o_first = up, o_acc = o_first + al(sizeof(int) * (nslots + 1));
+    const size_t o_coef = o_acc + al(sizeof(int) * P.jac.size()), o_end = o_coef + al(sizeof(double) * P.jac.size());
+    if (P.bwd) up = o_end;
+    const size_t o_part = up, b_part = P.bwd ? al(sizeof(double) * (size_t)nsweep * P.nacc * gx) : 0;
+    const size_t o_jac = o_part + b_part, b_jac = P.bwd ? sizeof(double) * (size_t)nsweep * nslots : 0;
+    std::vector<unsigned char> host(up, 0);
+    for (size_t i = 0; i < P.passes.size(); i++)
+        std::memcpy(host.data() + at[i], P.passes[i].blob.data(), P.passes[i].blob.size());
+    if (P.bwd) { // terms by slot
+        int *first = reinterpret_cast<int *>(host.data() + o_first), *ta = reinterpret_cast<int *>(host.data() + o_acc);
+        double *tc = reinterpret_cast<double *>(host.data() + o_coef);
+        for (const JacTerm &t : P.jac) first[t.slot + 1]++;
+        for (int s = 0; s < nslots; s++) first[s + 1] += first[s];
+        std::vector<int> next(first, first + nslots);
+        for (const JacTerm &t : P.jac) {
+            ta[next[t.slot]] = t.acc;
+            tc[next[t.slot]++] = t.coef * share;
+        }
+    }
+    PoolBuf buf(st);
+    PLK_CUDA(cudaMallocFromPoolAsync(&buf.p, o_jac + b_jac + 256, d->pool, st));
+    unsigned char *dev = buf.as<unsigned char>();
+    PLK_CUDA(cudaMemcpyAsync(dev, host.data(), up, cudaMemcpyHostToDevice, st));
+    Args a;
+    std::memset((void *)&a, 0, sizeof(a));
+    for (int y = 0; y < nsweep; y++) {
+        a.lam_src[y] = lam_src[y];
+        a.lam[y] = lam[y];
+        a.hl[y] = P.bwd ? hl[y] : nullptr;
+    }
+    a.T = P.T;
+    a.ntiles = ntiles;
+    a.nacc_all = P.nacc;
+    a.part = reinterpret_cast<double *>(dev + o_part);
+    const dim3 grid(gx, nsweep);
+    for (size_t i = 0; i < P.passes.size(); i++) {
+        const TileHdr &h = *reinterpret_cast<const TileHdr *>(P.passes[i].blob.data());
+        a.prog = dev + at[i];
+        a.prog_bytes = h.bytes;
+        a.nacc = h.nacc;
+        a.in_df = i > 0;
+        a.out_df = i + 1 < P.passes.size();
+        const size_t smem = smem_bytes(c64 ? 8 : 16, P.bwd, P.T, h.bytes, h.nacc, threads);
+        if (c64) PLK_TRY(launch_c64(P.bwd, a, grid, threads, smem, st));
+        else if (P.bwd) PLK_TRY(launch_c128_bwd(a, grid, threads, smem, st));
+        else PLK_TRY(launch_c128_fwd(a, grid, threads, smem, st));
+        for (int y = 0; y < nsweep; y++) a.lam_src[y] = lam[y];
+    }
+    if (P.bwd && nslots > 0) {
+        double *dj = reinterpret_cast<double *>(dev + o_jac);
+        k_tile_jac<<<dim3((nslots + 7) / 8, nsweep), 256, 0, st>>>(
+            a.part, gx, P.nacc, reinterpret_cast<const int *>(dev + o_first), reinterpret_cast<const int *>(dev + o_acc),
+            reinterpret_cast<const double *>(dev + o_coef), nslots, dj);
+        PLK_CHECK_LAUNCH();
+        PLK_CUDA(cudaMemcpyAsync(jac_host, dj, b_jac, cudaMemcpyDeviceToHost, st));
+        PLK_CUDA(cudaStreamSynchronize(st));
+    }
+    return PLK_OK;
+}
+
+// an op that the per-op path would accept
+static bool well_formed(plk_state s, const plk_op &op) {
+    if (op.gate <= PLK_GATE_IDENTITY || op.gate >= PLK_GATE_MATRIX) return false;
+    const int nw = plk_gate_num_wires(op.gate), np = plk_gate_num_params(op.gate);
+    if (nw > 0 ? op.num_wires != nw : op.num_wires < 1) return false;
+    if (op.num_params < np || (op.num_params > 0 && !op.params)) return false;
+    return check_wires(s, op.wires, op.num_wires) == PLK_OK;
+}
+
+static bool has_generator(int gate, int nw) {
+    GatePlan p;
+    return plan_generator(gate, nw, p) == PLK_OK;
+}
+
+static bool usable(plk_state s) {
+    return window_path_enabled() && (s->dtype == PLK_C64 || c128_use_df()) && s->nq >= kMaxRegBits && s->nq <= 32;
+}
+
+// The whole op list as passes; handled stays false when an op is not of this
+// path (dense matrices) or not well formed (the per-op path reports it).
+int apply_ops(plk_state s, const plk_op *ops, int nops, bool &handled) {
+    handled = false;
+    if (!usable(s) || nops < 4) return PLK_OK;
+    Compiler c(s->nq, false, options(s->nq, s->dtype, false));
+    Lowered L;
+    for (int i = 0; i < nops; i++) {
+        if (ops[i].gate == PLK_GATE_IDENTITY) continue;
+        L.v.clear();
+        if (!well_formed(s, ops[i]) || !lower_op(ops[i], s->nq, -1, L)) return PLK_OK;
+        c.add(L.v);
+    }
+    TileProgram P;
+    if (!c.compile(P)) return PLK_OK;
+    handled = true;
+    const void *src[1] = {s->data};
+    void *dst[1] = {s->data};
+    return run(P, s->dtype, s->device, s->stream, src, dst, nullptr, 1, 0, nullptr);
+}
+
+// Backward sweeps of all observables; lam is the working copy of the forward
+// state (overwritten by the last group of sweeps).
+int adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops, const int64_t *tp, int ntp,
+            double *jac, bool &handled) {
+    handled = false;
+    if (!usable(lam) || ntp <= 0 || nobs < 1) return PLK_OK;
+    int num_param_ops = 0;
+    for (int i = 0; i < nops; i++)
+        if (ops[i].num_params > 0) num_param_ops++;
+    // the reference's backward walk: ops in reverse until every trainable
+    // parameter is done (AdjointDiffKokkos.hpp:436-470)
+    Compiler c(lam->nq, true, options(lam->nq, lam->dtype, true));
+    Lowered L;
+    long current_param_idx = num_param_ops - 1;
+    int tp_it = ntp - 1, swept = 0;
+    for (int i = nops - 1; i >= 0 && tp_it >= 0; i--) {
+        const plk_op &op = ops[i];
+        if (op.num_params > 1) return PLK_OK; // rejected by the reference; the per-op path reports it
+        const bool trainable = op.num_params > 0 && current_param_idx == tp[tp_it];
+        if (op.gate != PLK_GATE_IDENTITY) {
+            L.v.clear();
+            if (!well_formed(lam, op) || (trainable && !has_generator(op.gate, op.num_wires)) ||
+                !lower_op(op, lam->nq, trainable ? tp_it : -1, L))
+                return PLK_OK;
+            invert(L.v);
+            c.add(L.v);
+            swept++;
+        } else if (trainable) {
+            return PLK_OK;
+        }
+        if (trainable) tp_it--;
+        if (op.num_params > 0) current_param_idx--;
+    }
+    TileProgram P;
+    if (!c.compile(P) || P.passes.empty()) return PLK_OK;
+    // 4 state moves per pass and observable, against 2 (1 + nobs) per op for
+    // the op-at-a-time kernel that carries every H lambda along
+    if (nobs > 1 && 4.0 * nobs * P.passes.size() > 2.0 * (1.0 + nobs) * swept) return PLK_OK;
+    // several sweeps start from lambda: each works on its own copy
+    const size_t bytes = lam->length * amp_bytes(lam->dtype);
+    int group = std::min(nobs, kMaxSweeps);
+    PoolBuf copies(lam->stream);
+    if (nobs > 1) {
+        const size_t most = (size_t)2 << 30;
+        group = (int)std::min<size_t>(group, std::max<size_t>(1, most / bytes));
+        if (pool_alloc(lam->device, &copies.p, bytes * group, lam->stream) != PLK_OK) {
+            // no room for a copy of lambda: the op-at-a-time path needs none
+            cudaGetLastError();
+            set_error(std::string());
+            return PLK_OK;
+        }
+    }
+    handled = true;
+    for (int o0 = 0; o0 < nobs; o0 += group) {
+        const int n = std::min(group, nobs - o0);
+        const void *src[kMaxSweeps];
+        void *dst[kMaxSweeps], *h[kMaxSweeps];
+        for (int y = 0; y < n; y++) {
+            src[y] = lam->data;
+            h[y] = hls[o0 + y]->data;
+            dst[y] = nobs == 1 ? lam->data : copies.as<char>() + bytes * y;
+        }
+        PLK_TRY(run(P, lam->dtype, lam->device, lam->stream, src, dst, h, n, ntp, jac + (size_t)o0 * ntp));
+    }
+    if (nobs > 1) // lambda ends as the swept state, as with one observable
+        PLK_CUDA(cudaMemcpyAsync(lam->data, copies.p, bytes, cudaMemcpyDeviceToDevice, lam->stream));
+    return PLK_OK;
+}
+
+} // namespace tile
+} // namespace plk

@@ -276,9 +276,16 @@ static int run_program(plk_state lam, plk_state hl, const StateProgram &P, bool 
 
 bool window_path_enabled() { return g_window_path.load() != 0; }
 
+namespace tile { // tile_sweep.cu: everything but dense matrices
+int apply_ops(plk_state s, const plk_op *ops, int nops, bool &handled);
+int adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops, const int64_t *tp, int ntp,
+            double *jac, bool &handled);
+} // namespace tile
+
 // Forward: the whole op list through windows (complex64).
 int window_apply_ops(plk_state s, const plk_op *ops, int nops, bool &handled) {
-    handled = false;
+    PLK_TRY(tile::apply_ops(s, ops, nops, handled));
+    if (handled) return PLK_OK;
     if (!window_path_enabled() || (s->dtype != PLK_C64 && !c128_use_df()) || nops < 4 || s->nq < 6 || s->nq > 32)
         return PLK_OK;
     std::vector<XOp> xs;
@@ -387,7 +394,8 @@ static int window_adjoint_concurrent(plk_state lam, plk_state *hls, int nobs, co
 // `lam` is the working copy of the forward state (overwritten).
 int window_adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops, const int64_t *tp, int ntp,
                    double *jac, bool &handled) {
-    handled = false;
+    PLK_TRY(tile::adjoint(lam, hls, nobs, ops, nops, tp, ntp, jac, handled));
+    if (handled) return PLK_OK;
     if (!window_path_enabled() || (lam->dtype != PLK_C64 && !c128_use_df()) || lam->nq < 6 || lam->nq > 32 ||
         ntp <= 0)
         return PLK_OK;
