@@ -10,10 +10,13 @@
 // XOR-swizzled and the host picks lane bits whose slots fall into different
 // banks.
 //
-// A rotation runs as three shears, x -= t y, y += s x, x -= t y with
+// complex64 runs a rotation as three shears, x -= t y, y += s x, x -= t y with
 // t = tan(angle / 2) <= 0.42: every step updates a register in place, so the
 // branches around a step need no register moves (the two-output form cost one
-// move per amplitude and step, a quarter of all instructions).
+// move per amplitude and step, a quarter of all instructions).  complex128 is
+// bound by the FP32 pipe, where a product and sum of double-floats takes 12
+// packed instructions: it runs [[1, -t], [t, 1]], two of them per pair, and
+// leaves the cosine to the next phase table.
 //
 // complex64: an amplitude is one packed FP32 pair (re, im), so a rotation is
 // three .f32x2 instructions per pair of amplitudes.  complex128: the tile holds
@@ -128,15 +131,14 @@ struct RotC64 {
         x = f2x_fma(nt, y, x);
     }
 };
+// (x, y) <- (x - t y, y + t x); the factor cos is in a phase table
 struct RotC128 {
-    f2x th, nth, tl, sh, nsh, sl;
-    __device__ __forceinline__ explicit RotC128(float4 k)
-        : th(f2x_dup(k.x)), nth(f2x_dup(-k.x)), tl(f2x_dup(k.y)), sh(f2x_dup(k.z)), nsh(f2x_dup(-k.z)),
-          sl(f2x_dup(k.w)) {}
+    f2x th, nth, tl;
+    __device__ __forceinline__ explicit RotC128(float4 k) : th(f2x_dup(k.x)), nth(f2x_dup(-k.x)), tl(f2x_dup(k.y)) {}
     __device__ __forceinline__ void operator()(AmpC128::V &x, AmpC128::V &y) const {
+        const AmpC128::V x0 = x;
         pdf_msub(th, nth, tl, y.h, y.l, x.h, x.l);
-        pdf_mac(sh, nsh, sl, x.h, x.l, y.h, y.l);
-        pdf_msub(th, nth, tl, y.h, y.l, x.h, x.l);
+        pdf_mac(th, nth, tl, x0.h, x0.l, y.h, y.l);
     }
 };
 // (x, y) <- (c x - s y, s x + c y): any angle, and exact for quarter turns
@@ -544,19 +546,21 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_tile(const __grid_constant__ 
                 }
             const uint32_t o = q.lo[lane] ^ q.hi[warp] ^ q.xorc ^ ev;
             const uint32_t r0 = q.rcol[0], r1 = q.rcol[1], r2 = q.rcol[2], r3 = q.rcol[3];
+            const uint32_t r01 = r0 ^ r1, r23 = r2 ^ r3; // one three-input operation per slot
             auto slot = [&](int j) {
-                return o ^ ((j & 1) ? r0 : 0u) ^ ((j & 2) ? r1 : 0u) ^ ((j & 4) ? r2 : 0u) ^ ((j & 8) ? r3 : 0u);
+                return o ^ ((j & 3) == 3 ? r01 : (j & 1) ? r0 : (j & 2) ? r1 : 0u) ^
+                       ((j & 12) == 12 ? r23 : (j & 4) ? r2 : (j & 8) ? r3 : 0u);
             };
             V v[NA], h[NA];
             if (r == 0) {
                 const TileIndex &x = index[hd.load_idx];
                 const uint32_t g = gev ^ x.lo[lane] ^ x.hi[warp] ^ x.c;
-                const uint32_t g0 = x.r[0], g1 = x.r[1], g2 = x.r[2], g3 = x.r[3];
+                const uint32_t g0 = x.r[0], g1 = x.r[1], g2 = x.r[2], g3 = x.r[3], g01 = g0 ^ g1, g23 = g2 ^ g3;
                 const void *lam = a.lam_src[blockIdx.y], *hl = a.hl[blockIdx.y];
 #pragma unroll
                 for (int j = 0; j < NA; j++) {
-                    const uint32_t i = g ^ ((j & 1) ? g0 : 0u) ^ ((j & 2) ? g1 : 0u) ^ ((j & 4) ? g2 : 0u) ^
-                                       ((j & 8) ? g3 : 0u);
+                    const uint32_t i = g ^ ((j & 3) == 3 ? g01 : (j & 1) ? g0 : (j & 2) ? g1 : 0u) ^
+                                       ((j & 12) == 12 ? g23 : (j & 4) ? g2 : (j & 8) ? g3 : 0u);
                     v[j] = load_amp(lam, i, a.in_df, V{});
                     if (BWD) h[j] = load_amp(hl, i, a.in_df, V{});
                 }
@@ -642,12 +646,12 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_tile(const __grid_constant__ 
                     if (base >> events[k].bit & 1u) go ^= events[k].gmask;
                 const TileIndex &x = index[hd.store_idx];
                 const uint32_t g = go ^ x.lo[lane] ^ x.hi[warp] ^ x.c;
-                const uint32_t g0 = x.r[0], g1 = x.r[1], g2 = x.r[2], g3 = x.r[3];
+                const uint32_t g0 = x.r[0], g1 = x.r[1], g2 = x.r[2], g3 = x.r[3], g01 = g0 ^ g1, g23 = g2 ^ g3;
                 void *lam = a.lam[blockIdx.y], *hl = a.hl[blockIdx.y];
 #pragma unroll
                 for (int j = 0; j < NA; j++) {
-                    const uint32_t i = g ^ ((j & 1) ? g0 : 0u) ^ ((j & 2) ? g1 : 0u) ^ ((j & 4) ? g2 : 0u) ^
-                                       ((j & 8) ? g3 : 0u);
+                    const uint32_t i = g ^ ((j & 3) == 3 ? g01 : (j & 1) ? g0 : (j & 2) ? g1 : 0u) ^
+                                       ((j & 12) == 12 ? g23 : (j & 4) ? g2 : (j & 8) ? g3 : 0u);
                     store_amp(lam, i, a.out_df, v[j]);
                     if (BWD) store_amp(hl, i, a.out_df, h[j]);
                 }

@@ -8,9 +8,17 @@
 namespace plk {
 namespace tile {
 
-// register bits, CTA threads (2^(largest T - R)) and CTAs per SM
-constexpr int kRegsC64Fwd = 4, kThreadsC64Fwd = 512, kCtasC64Fwd = 2;
-constexpr int kRegsC64Bwd = 4, kThreadsC64Bwd = 256, kCtasC64Bwd = 2;
+// Register bits, CTA threads (2^(largest T - R)) and CTAs per SM.  All shapes
+// fill the register file; smaller CTAs drift apart, so that one's memory phase
+// runs under another's arithmetic, larger ones need fewer passes.  Measured
+// (27-qubit QAOA, complex64 forward): 512 x 2 9.78 ms, 256 x 4 9.54, 128 x 8
+// 9.18.  26-qubit gradient, complex64 backward: 256 x 2 41.9 ms, 128 x 4 40.0,
+// R = 3 512 x 2 44.7.  25-qubit circuit, complex128 forward: 256 x 2 8.23 ms,
+// 128 x 4 8.16, 64 x 8 8.81, R = 3 512 x 2 8.65.  20-qubit Jacobian, complex128
+// backward: R = 3 256 x 2 32.8 ms, 128 x 4 36.9; R = 4 (its code overflows the
+// instruction cache) 128 x 2 36.0, 64 x 4 35.3.
+constexpr int kRegsC64Fwd = 4, kThreadsC64Fwd = 128, kCtasC64Fwd = 8;
+constexpr int kRegsC64Bwd = 4, kThreadsC64Bwd = 128, kCtasC64Bwd = 4;
 constexpr int kRegsC128Fwd = 4, kThreadsC128Fwd = 256, kCtasC128Fwd = 2;
 constexpr int kRegsC128Bwd = 3, kThreadsC128Bwd = 256, kCtasC128Bwd = 2;
 constexpr size_t kMaxBlob = 20480;

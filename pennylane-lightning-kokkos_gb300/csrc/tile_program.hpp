@@ -7,8 +7,10 @@
 //   RX = S^dag RY S, IsingXX = CX (RX x 1) CX, IsingYY = S S (XX) S^dag S^dag,
 //   SingleExcitation = CX(a,b) controlled-RY(a | b = 1) CX(a,b), and so on;
 // runs of one-wire gates on one wire are multiplied and split as
-// diag RY diag (|s| <= c: a half turn is taken out as an X), a rotation running
-// as three shears in place.  Index maps move no data: a tile keeps the linear map over
+// diag RY diag (|s| <= c: a half turn is taken out as an X).  complex64 runs the
+// rotation as three shears in place; complex128 as [[1, -t], [t, 1]], t = s / c,
+// whose factor c goes into the next phase table (two double-float products per
+// amplitude pair instead of three).  Index maps move no data: a tile keeps the linear map over
 // GF(2) from logical index to shared-memory slot and composes CNOTs into it; a
 // CNOT whose control lies outside the tile flips a constant of that map.
 //
@@ -59,7 +61,7 @@ enum SpecialKind : uint8_t { TS_NONE = 0, TS_CRY = 1, TS_DIAG = 2, TS_PAR = 3 };
 // Order within a stage: sums of the table, table, rotations by ascending bit,
 // special step.
 struct alignas(16) TileStage { // 144 bytes
-    float rot[4][4]; // bit b: the shears t, s as t.hi t.lo s.hi s.lo
+    float rot[4][4]; // bit b: complex64 the shears t, s as t.hi t.lo s.hi s.lo; complex128 t = s / c as t.hi t.lo
     int16_t acc_y[4], acc_x[4]; // accumulators of Im <h|Y|v>, Im <h|X|v> (-1: none)
     uint8_t ry;      // bits that turn
     uint8_t table;   // bit 0: sums wanted (zsel), bit 1: phases to apply
@@ -526,6 +528,8 @@ class Compiler {
             if (indeg_[i] == 0) ready.push_back(i);
         deg_.assign(units_.size(), 0);
         in_.assign(units_.size(), 0);
+        pend_ = 1;
+        last_table_ = Table{};
         size_t done = 0;
         std::vector<int> sel;
         std::vector<JacTerm> jac;
@@ -535,8 +539,14 @@ class Compiler {
             if (sel.empty()) return false;
             TilePass pass;
             int nacc = 0;
+            const double pend = pend_;
+            const Table last_table = last_table_;
             for (;;) {
                 jac.clear();
+                pend_ = pend;
+                last_table_ = last_table;
+                pass_ = (int)P.passes.size();
+                jac0_ = P.jac.size();
                 if (!build_pass(sel, bits, P.nacc, pass, jac, nacc)) return false;
                 if (pass.blob.size() <= o_.max_blob || sel.size() <= 4) break;
                 sel.resize(sel.size() * 3 / 4);
@@ -552,6 +562,19 @@ class Compiler {
             P.jac.insert(P.jac.end(), jac.begin(), jac.end());
             P.passes.push_back(std::move(pass));
         }
+        if (pend_ != 1) { // rotations after the last table: their factors go into it
+            if (last_table_.pass < 0) return false;
+            TilePass &p = P.passes[last_table_.pass];
+            float *f = reinterpret_cast<float *>(
+                p.blob.data() + reinterpret_cast<const TileHdr *>(p.blob.data())->off_tab + (size_t)last_table_.entry * 16);
+            for (int k = 0; k < 4 << R_; k += 4)
+                for (int q = 0; q < 2; q++) {
+                    const double x = ((double)f[k + q] + (double)f[k + 2 + q]) * pend_;
+                    f[k + q] = (float)x;
+                    f[k + 2 + q] = (float)(x - (double)f[k + q]);
+                }
+            for (size_t i = last_table_.jac; i < P.jac.size(); i++) P.jac[i].coef /= pend_ * pend_;
+        }
         return true;
     }
 
@@ -566,6 +589,16 @@ class Compiler {
     std::vector<int> indeg_;
     std::vector<int> deg_;  // scratch: in-degrees inside a selection
     std::vector<char> in_;  // scratch: members of a selection
+    // complex128: the state is pend_ times what the sweep holds
+    double pend_ = 1;
+    struct Table { // the last phase table: pass, first entry, Jacobian terms before it
+        int pass = -1;
+        uint32_t entry = 0;
+        size_t jac = 0;
+    } last_table_;
+    int pass_ = 0;
+    size_t jac0_ = 0;
+    bool scaled() const { return o_.amp_bytes == 16; }
 
     static int popc(uint32_t x) { return __builtin_popcount(x); }
     static void insert_sorted(std::vector<int> &v, int x) { v.insert(std::lower_bound(v.begin(), v.end(), x), x); }
@@ -750,6 +783,22 @@ class Compiler {
             if (flip) push_x(t);
         }
         prims_.clear();
+        if (scaled()) { // some phase table has to take the rotations' factors
+            bool turns = false, tables = false;
+            for (const Unit &u : units_)
+                if (u.kind == P_U1) {
+                    turns = true;
+                    tables = tables || u.has_a || u.has_b;
+                }
+            if (turns && !tables) {
+                Unit u;
+                u.kind = u.p.kind = P_DIAG;
+                u.p.K = 1;
+                u.p.d[0] = u.p.d[1] = 1;
+                u.bits = 1;
+                push(std::move(u));
+            }
+        }
         if (!near(g, 1)) { // into the first table there is
             for (Unit &u : units_) {
                 if (u.kind == P_DIAG || u.kind == P_PAR) {
@@ -1085,7 +1134,7 @@ class Compiler {
     }
 
     bool emit_round(Out &o, const std::vector<Step> &st, uint32_t regs, int acc0, std::vector<JacTerm> &jac,
-                    int &nacc) const {
+                    int &nacc) {
         if (o.rounds.empty()) { // reads the state
             const uint32_t c = o.xc;
             std::vector<uint32_t> col = o.col;
@@ -1109,7 +1158,7 @@ class Compiler {
         bool want_index = false;
         auto acc = [&](const Terms &t) -> int16_t {
             if (t.empty()) return -1;
-            for (const auto &e : t) jac.push_back(JacTerm{e.first, acc0 + nacc, e.second});
+            for (const auto &e : t) jac.push_back(JacTerm{e.first, acc0 + nacc, e.second * pend_ * pend_});
             return (int16_t)nacc++;
         };
         auto reg_of = [&](int state_bit) {
@@ -1123,14 +1172,38 @@ class Compiler {
             return q;
         };
         TileStage cur;
+        const Unit *turn[4]; // rotations of the stage by bit
         bool any = false;
         auto reset = [&]() {
             std::memset(&cur, 0, sizeof(cur));
-            for (int i = 0; i < 4; i++) cur.acc_y[i] = cur.acc_x[i] = -1;
+            for (int i = 0; i < 4; i++) {
+                cur.acc_y[i] = cur.acc_x[i] = -1;
+                turn[i] = nullptr;
+            }
             cur.acc_z = cur.sacc = -1;
             any = false;
         };
+        // rotations run by ascending bit, each measured before it runs
+        auto turns = [&]() {
+            for (int b = 0; b < R_; b++) {
+                if (!turn[b]) continue;
+                const Unit &u = *turn[b];
+                cur.ry |= (uint8_t)(1u << b);
+                if (scaled()) {
+                    put2(cur.rot[b], u.p.s / u.p.c);
+                } else {
+                    put2(cur.rot[b], u.p.s / (1.0 + u.p.c));
+                    put2(cur.rot[b] + 2, u.p.s);
+                }
+                cur.acc_y[b] = acc(u.gy);
+                cur.acc_x[b] = acc(u.gx);
+                cur.sums |= (uint8_t)((cur.acc_y[b] >= 0 ? 1 : 0) | (cur.acc_x[b] >= 0 ? 2 : 0));
+                if (scaled()) pend_ *= u.p.c;
+                turn[b] = nullptr;
+            }
+        };
         auto flush = [&]() {
+            turns();
             if (any) o.stages.push_back(cur);
             reset();
         };
@@ -1140,11 +1213,13 @@ class Compiler {
             if (s.kind == SK_TAB) {
                 if (any) flush();
                 any = true;
-                if (!s.f.empty()) {
+                const double scale = pend_;
+                if (!s.f.empty() || pend_ < 1.0 / 256) {
                     cur.table |= 2;
                     cur.tab = (uint16_t)tab_pos(o);
                     cplx e[kMaxAmps];
-                    for (int j = 0; j < amps; j++) e[j] = 1;
+                    for (int j = 0; j < amps; j++) e[j] = pend_;
+                    pend_ = 1;
                     for (const Factor &f : s.f) {
                         if (!f.u) {
                             const int i = reg_of(f.bit);
@@ -1175,21 +1250,18 @@ class Compiler {
                             cur.zsel |= (uint16_t)(1u << z[i].first);
                             nacc++;
                         }
-                        jac.push_back(JacTerm{z[i].second->slot, acc0 + nacc - 1, z[i].second->coef});
+                        jac.push_back(JacTerm{z[i].second->slot, acc0 + nacc - 1, z[i].second->coef * scale * scale});
                     }
                 }
+                if (cur.table & 2) last_table_ = Table{pass_, cur.tab, jac0_ + jac.size()};
             } else if (s.kind == SK_RY) {
                 const int b = reg_of(s.u->p.t);
-                if (cur.special || (cur.ry >> b & 1)) flush();
+                if (cur.special || turn[b]) flush();
                 any = true;
-                cur.ry |= (uint8_t)(1u << b);
-                put2(cur.rot[b], s.u->p.s / (1.0 + s.u->p.c));
-                put2(cur.rot[b] + 2, s.u->p.s);
-                cur.acc_y[b] = acc(s.u->gy);
-                cur.acc_x[b] = acc(s.u->gx);
-                cur.sums |= (uint8_t)((cur.acc_y[b] >= 0 ? 1 : 0) | (cur.acc_x[b] >= 0 ? 2 : 0));
+                turn[b] = s.u;
             } else {
                 if (cur.special) flush();
+                turns();
                 any = true;
                 const Unit &u = *s.u;
                 if (s.kind == SK_CRY) {
@@ -1332,6 +1404,14 @@ class Compiler {
                 place(st, u, regs);
             }
             for (int k = T_ - 1; k >= 0 && popc(regs) < R_; k--) regs |= 1u << o.tbits[k];
+            if (pend_ < 1.0 / 256) { // keep what the sweep holds within 2^12 of the state
+                bool table = false;
+                for (const Step &x : st) table = table || x.kind == SK_TAB;
+                if (!table) {
+                    st.insert(st.begin(), Step{});
+                    st.front().kind = SK_TAB;
+                }
+            }
             ok = !st.empty() && emit_round(o, st, regs, acc0, jac, nacc);
         }
         for (int i : sel) in_[i] = 0, deg_[i] = 0;

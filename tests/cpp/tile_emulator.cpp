@@ -141,9 +141,15 @@ extern "C" int tile_emulate(int nq, int T, int R, int low, int amp, int bwd, con
                                 if (st.acc_x[b] >= 0) acc[h.acc0 + st.acc_x[b]] += imdot(hx, y) + imdot(hy, x);
                                 for (int z = 0; z < 2; z++) {
                                     C &p = z ? hx : x, &u = z ? hy : y;
-                                    p -= tt * u;
-                                    u += ss * p;
-                                    p -= tt * u;
+                                    if (amp == 16) { // complex128: [[1, -t], [t, 1]]
+                                        const C p0 = p;
+                                        p -= tt * u;
+                                        u += tt * p0;
+                                    } else {
+                                        p -= tt * u;
+                                        u += ss * p;
+                                        p -= tt * u;
+                                    }
                                 }
                             }
                         }
