@@ -12,6 +12,7 @@
 
 #include "df.cuh"
 #include "gate_ops.cuh"
+#include "pauli_tile.cuh"
 #include "reduce.cuh"
 #include "expval_diag.cuh"
 
@@ -252,20 +253,6 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // ---------------------------------------------------------- Pauli words --
-// A Pauli word P acts as P|k> = i^ny (-1)^popcount(k & z) |k ^ x>, with x the
-// X/Y positions, z the Y/Z positions, ny the number of Y letters.  Terms that
-// share x form one group; a group costs one pass over the state.
-struct PauliTerm {
-    uint64_t z;
-    double cr, ci;           // c_j * i^ny
-    float crh, crl, cih, cil; // the same, split for the FP32-pipe accumulation
-};
-
-struct PauliGroup {
-    uint64_t x;
-    int first, count;
-};
-
 static int build_pauli_groups(plk_state s, int nterms, const double *coeffs, const int64_t *offsets,
                               const int64_t *wires, const char *paulis, std::vector<PauliGroup> &groups,
                               std::vector<PauliTerm> &terms) {
@@ -830,14 +817,24 @@ static int free_csr(plk_state s, CsrDev &c) {
 }
 
 template <class T>
-static int pauli_expval_impl(plk_state s, const std::vector<PauliGroup> &groups, const std::vector<PauliTerm> &terms,
+static int pauli_expval_impl(plk_state s, const std::vector<PauliGroup> &all, const std::vector<PauliTerm> &terms,
                              double *out) {
+    for (const PauliGroup &g : all)
+        if (sizeof(PauliTerm) * g.count > 48 * 1024)
+            PLK_FAIL(PLK_ERR_UNSUPPORTED, "too many Pauli terms share one X pattern");
+    // most groups on tiles, several per pass over the state; the others one pass each
+    std::vector<PauliGroup> groups;
+    double total = 0.0;
+    PLK_TRY(pauli_tile_expval(s, all, terms, groups, total));
+    if (groups.empty()) {
+        *out = total;
+        return PLK_OK;
+    }
     PoolBuf dt_buf(s->stream);
     PLK_TRY(pool_alloc(s->device, &dt_buf.p, sizeof(PauliTerm) * std::max<size_t>(terms.size(), 1), s->stream));
     PauliTerm *dt = dt_buf.as<PauliTerm>();
     PLK_CUDA(cudaMemcpyAsync(dt, terms.data(), sizeof(PauliTerm) * terms.size(), cudaMemcpyHostToDevice, s->stream));
     // each group's partial lands in d_result[gi % kMaxRedValues]; fetch in chunks
-    double total = 0.0;
     auto &w = s->ws;
     std::vector<double> vals(groups.size());
     for (size_t gi = 0; gi < groups.size(); gi++) {
@@ -848,7 +845,6 @@ static int pauli_expval_impl(plk_state s, const std::vector<PauliGroup> &groups,
             pmask_lo = (1ULL << p) - 1;
         }
         const size_t smem = sizeof(PauliTerm) * g.count;
-        if (smem > 48 * 1024) PLK_FAIL(PLK_ERR_UNSUPPORTED, "too many Pauli terms share one X pattern");
         const int grid = red_grid_k(s, k_expval_pauli<T>, g.x ? s->length >> 1 : s->length, smem);
         k_expval_pauli<T><<<grid, kThreads, smem, s->stream>>>((const c2_t<T> *)s->data, s->length, g.x, pmask_lo,
                                                               dt + g.first, g.count, w.d_partials,
@@ -865,9 +861,16 @@ static int pauli_expval_impl(plk_state s, const std::vector<PauliGroup> &groups,
 }
 
 template <class T>
-static int pauli_apply_impl(plk_state outs, plk_state ins, const std::vector<PauliGroup> &groups,
+static int pauli_apply_impl(plk_state outs, plk_state ins, const std::vector<PauliGroup> &all,
                             const std::vector<PauliTerm> &terms) {
     cudaStream_t st = outs->stream;
+    std::vector<PauliGroup> groups;
+    bool accumulate = false;
+    PLK_TRY(pauli_tile_apply(outs, ins, all, terms, groups, accumulate));
+    if (groups.empty() && accumulate) {
+        PLK_CUDA(cudaStreamSynchronize(st)); // the caller may free `ins` on return
+        return PLK_OK;
+    }
     PoolBuf dt_buf(st);
     PLK_TRY(pool_alloc(outs->device, &dt_buf.p, sizeof(PauliTerm) * std::max<size_t>(terms.size(), 1), st));
     PauliTerm *dt = dt_buf.as<PauliTerm>();
@@ -876,14 +879,18 @@ static int pauli_apply_impl(plk_state outs, plk_state ins, const std::vector<Pau
     for (size_t g0 = 0; g0 < groups.size(); g0 += kPauliGroupsPerPass) {
         PauliPass pass;
         pass.ngroups = (int)std::min<size_t>(kPauliGroupsPerPass, groups.size() - g0);
-        pass.accumulate = g0 > 0;
+        pass.accumulate = g0 > 0 || accumulate;
         for (int i = 0; i < pass.ngroups; i++) {
             pass.x[i] = groups[g0 + i].x;
             pass.first[i] = groups[g0 + i].first;
             pass.count[i] = groups[g0 + i].count;
         }
-        const int t_lo = pass.first[0];
-        const int t_cnt = pass.first[pass.ngroups - 1] + pass.count[pass.ngroups - 1] - t_lo;
+        int t_lo = pass.first[0], t_hi = 0;
+        for (int i = 0; i < pass.ngroups; i++) {
+            t_lo = std::min(t_lo, pass.first[i]);
+            t_hi = std::max(t_hi, pass.first[i] + pass.count[i]);
+        }
+        const int t_cnt = t_hi - t_lo;
         const size_t smem = sizeof(PauliTerm) * (size_t)t_cnt;
         const int in_smem = smem <= 48 * 1024 ? 1 : 0;
         // one resident wave of blocks, each walking its tiles in order

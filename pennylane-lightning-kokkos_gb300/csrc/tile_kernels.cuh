@@ -484,6 +484,27 @@ __device__ __forceinline__ void step_cry(typename A::V (&v)[1 << R], typename A:
     }
 }
 
+// A double as a normalised double-float, both parts rounded to nearest.  The
+// truncating split of df.cuh leaves a low part of up to 2^-23 of the high part,
+// always of its sign, and what it cuts off and the low parts' dropped products
+// add up to a bias of about 2^-48 of a sum's magnitudes (seen in energies whose
+// words nearly cancel: 8e-13 against 8e-14).
+__device__ __forceinline__ DF df_split_near(double x) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    const unsigned hw = (unsigned)(u >> 32), lw = (unsigned)u, sign = hw & 0x80000000u;
+    const int ef = (int)((hw >> 20) & 0x7ffu) - 896, el = ef - 23; // float exponents of hi and of its last place
+    const unsigned top = ((hw & 0xfffffu) << 3) | (lw >> 29);
+    const unsigned next = ((lw & 0x1fffffffu) + 32u) >> 6; // up to 2^23
+    const float hi = (ef >= 1 && ef <= 254) ? __uint_as_float(sign | ((unsigned)ef << 23) | top) : 0.0f;
+    float lo = 0.0f;
+    if (el >= 1 && el <= 253) { // (1 + next / 2^23) 2^E - 2^E, exact
+        const float f = __uint_as_float(((unsigned)el << 23) + next), g = __uint_as_float((unsigned)el << 23);
+        lo = __uint_as_float(__float_as_uint(__fsub_rn(f, g)) | sign);
+    }
+    const float s = __fadd_rn(hi, lo);
+    return {s, __fsub_rn(lo, __fsub_rn(s, hi))};
+}
+
 // state buffers: complex128 holds doubles outside a sweep and double-float
 // pairs between its passes
 __device__ __forceinline__ f2x load_amp(const void *p, uint32_t i, int, f2x) {
@@ -492,7 +513,8 @@ __device__ __forceinline__ f2x load_amp(const void *p, uint32_t i, int, f2x) {
 __device__ __forceinline__ AmpC128::V load_amp(const void *p, uint32_t i, int df, AmpC128::V) {
     const ulonglong2 a = __ldcg(static_cast<const ulonglong2 *>(p) + i);
     if (df) return {a.x, a.y};
-    const DF re = df_split(__longlong_as_double((long long)a.x)), im = df_split(__longlong_as_double((long long)a.y));
+    const DF re = df_split_near(__longlong_as_double((long long)a.x));
+    const DF im = df_split_near(__longlong_as_double((long long)a.y));
     return {f2x_pack(re.hi, im.hi), f2x_pack(re.lo, im.lo)};
 }
 __device__ __forceinline__ void store_amp(void *p, uint32_t i, int, f2x v) {

@@ -1,0 +1,82 @@
+"""GPU: Pauli sums on tiles (expectation value and application) against dense
+numpy evaluation, at sizes where tiles change (fewer amplitudes than a block
+holds, one tile, several) and for words that share an X pattern, have none, or
+are too wide for a tile.
+
+Tolerances, relative to the sum of |coefficients|: complex128 1e-12
+(double-float sums, 2^-45 per product, random signs); complex64 2e-6 (2^-24 per
+amplitude of a normalised state, eight products per single-precision sum).
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from abi import State, f64, i64
+from pennylane_lightning_kokkos import _native as N
+from test_oracle_golden import rand_state
+
+pytestmark = pytest.mark.gpu
+
+TOL = {N.PLK_C64: 2e-6, N.PLK_C128: 1e-12}
+
+
+def dense(psi, nq, words):
+    out = np.zeros_like(psi)
+    idx = np.arange(1 << nq)
+    for c, wires, letters in words:
+        x = z = ny = 0
+        for w, l in zip(wires, letters):
+            bit = 1 << (nq - 1 - w)
+            x |= bit if l in "XY" else 0
+            z |= bit if l in "YZ" else 0
+            ny += l == "Y"
+        par = np.array([bin(int(k)).count("1") & 1 for k in range(1 << 8)])
+        src = idx ^ x
+        s = src & z
+        sign = 1 - 2 * (par[s & 255] ^ par[(s >> 8) & 255])
+        out += c * (1j) ** ny * sign * psi[src]
+    return out
+
+
+def words_for(nq, rng, kind):
+    words = []
+    for k in range(40):
+        if kind == "shared": # few X patterns, many sign patterns
+            wires = list(range(min(nq, 4)))
+            letters = "".join(rng.choice(["XXYZ", "YYXI", "ZZII", "IZZI"])[: len(wires)])
+            extra = [int(w) for w in rng.choice(nq, 2, replace=False) if w >= len(wires)]
+            wires, letters = wires + extra, letters + "Z" * len(extra)
+        else:
+            wt = int(rng.integers(1, min(nq, 5) + 1)) if kind == "narrow" else int(rng.integers(1, nq + 1))
+            wires = [int(w) for w in rng.choice(nq, wt, replace=False)]
+            letters = "".join(str(x) for x in rng.choice(list("XYZ"), wt))
+        words.append((float(rng.standard_normal()), wires, letters))
+    return words
+
+
+@pytest.mark.parametrize("dtype", [N.PLK_C64, N.PLK_C128])
+@pytest.mark.parametrize("kind", ["narrow", "wide", "shared"])
+@pytest.mark.parametrize("nq", [4, 5, 8, 9, 11, 12, 13, 15])
+def test_pauli_sum(nq, kind, dtype):
+    rng = np.random.default_rng(31 * nq + len(kind))
+    psi = rand_state(nq, rng)
+    words = words_for(nq, rng, kind)
+    s, o = State.from_array(psi, dtype), State(nq, dtype)
+    ref = dense(s.get().astype(np.complex128), nq, words)
+    c, cp = f64([w[0] for w in words])
+    off, offp = i64(np.cumsum([0] + [len(w[1]) for w in words]))
+    wi, wp = i64([x for w in words for x in w[1]])
+    letters = "".join(w[2] for w in words).encode()
+    scale = float(np.sum(np.abs(c)))
+    v = C.c_double()
+    N.check(N.lib.plk_expval_pauli_sum(s.h, len(words), cp, offp, wp, letters, C.byref(v)))
+    want = float(np.vdot(s.get().astype(np.complex128), ref).real)
+    assert abs(v.value - want) < TOL[dtype] * scale
+    first = v.value
+    N.check(N.lib.plk_expval_pauli_sum(s.h, len(words), cp, offp, wp, letters, C.byref(v)))
+    assert v.value == first
+    N.check(N.lib.plk_apply_pauli_sum(o.h, s.h, len(words), cp, offp, wp, letters))
+    np.testing.assert_allclose(o.get(), ref, atol=TOL[dtype] * scale, rtol=0)
+    s.close()
+    o.close()
