@@ -22,7 +22,6 @@ int plan_gate(int gate, int nw, bool inv, const double *prm, int np, GatePlan &p
 int apply_matrix_impl(plk_state s, const double *matrix, const int64_t *wires, int nw, bool adj);
 
 int fetch_results(plk_state s, int nv, double *out) {
-    PLK_CUDA(cudaMemcpyAsync(s->ws.h_result, s->ws.d_result, sizeof(double) * nv, cudaMemcpyDeviceToHost, s->stream));
     PLK_CUDA(cudaStreamSynchronize(s->stream));
     std::memcpy(out, s->ws.h_result, sizeof(double) * nv);
     return PLK_OK;

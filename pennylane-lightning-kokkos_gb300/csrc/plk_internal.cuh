@@ -94,7 +94,7 @@ constexpr int kMaxRedValues = 64; // values reduced together in one pass
 // ----------------------------------------------------------------------------
 struct Workspace {
     double *d_partials = nullptr;   // [kMaxRedValues][kMaxRedBlocks]
-    double *d_result = nullptr;     // [kMaxRedValues]
+    double *d_result = nullptr;     // [kMaxRedValues]: h_result, written by the kernels themselves
     unsigned int *d_counter = nullptr;
     double *h_result = nullptr;     // pinned [kMaxRedValues]
 };
@@ -126,14 +126,13 @@ int device_sm_count(int device);
 // this kernel (a whole number per SM, so there is no partial last wave),
 // at most kMaxRedBlocks and no more than the work needs.  A function of the
 // kernel, the device and the size only, so the partial-sum order is fixed.
+// CTAs of a kernel that fit on an SM (the runtime's answer, kept per thread:
+// the query costs microseconds, a small reduction not much more).
+int resident_ctas(const void *kernel, size_t dyn_smem);
 template <class Kern>
 int red_grid_k(const plk_state_s *s, Kern kernel, uint64_t work_items, size_t dyn_smem = 0) {
     const int sms = device_sm_count(s->device);
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kThreads, dyn_smem) != cudaSuccess || occ < 1) {
-        cudaGetLastError();
-        occ = 1;
-    }
+    const int occ = resident_ctas(reinterpret_cast<const void *>(kernel), dyn_smem);
     int per_sm = kMaxRedBlocks / (sms > 0 ? sms : 1);
     if (per_sm > occ) per_sm = occ;
     if (per_sm < 1) per_sm = 1;

@@ -52,8 +52,8 @@ __device__ __forceinline__ void block_reduce_finish(double (&acc)[NV], double *_
 // Only the first `nvalid` results are written (NV may be a rounded-up
 // template size).
 
-// Copy `nv` reduced values to the host (pinned staging), synchronizing the
-// state's stream.
+// Waits for the state's stream and takes `nv` reduced values from the pinned
+// buffer that the kernels wrote.
 int fetch_results(plk_state s, int nv, double *out);
 
 } // namespace plk

@@ -121,6 +121,27 @@ int device_sm_count(int device) {
     return d->sm_count;
 }
 
+int resident_ctas(const void *kernel, size_t dyn_smem) {
+    struct Entry {
+        const void *kernel;
+        size_t smem;
+        int device, ctas;
+    };
+    thread_local std::vector<Entry> known;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    for (const Entry &e : known)
+        if (e.kernel == kernel && e.smem == dyn_smem && e.device == dev) return e.ctas;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kThreads, dyn_smem) != cudaSuccess || occ < 1) {
+        cudaGetLastError();
+        return 1;
+    }
+    if (known.size() >= 256) known.clear(); // sizes of dynamic shared memory vary with the caller's terms
+    known.push_back(Entry{kernel, dyn_smem, dev, occ});
+    return occ;
+}
+
 int red_grid(const plk_state_s *s, uint64_t work_items) {
     DeviceCtx *d = nullptr;
     if (device_ctx(s->device, &d) != PLK_OK) return 1;
@@ -304,15 +325,16 @@ PLK_API int plk_get_device_info(int device, plk_device_info *out) {
 }
 
 static int alloc_workspace(plk_state s) {
-    // partials, results and the ticket counter in one pool block
-    const size_t bp = sizeof(double) * kMaxRedValues * kMaxRedBlocks, br = sizeof(double) * kMaxRedValues;
+    // partials and the ticket counter in one pool block; results go straight to
+    // pinned host memory (a copy of its own costs a small call about 5 us)
+    const size_t bp = sizeof(double) * kMaxRedValues * kMaxRedBlocks;
     void *blk = nullptr;
-    PLK_TRY(pool_alloc(s->device, &blk, bp + br + 256, s->stream));
+    PLK_TRY(pool_alloc(s->device, &blk, bp + 256, s->stream));
     s->ws.d_partials = (double *)blk;
-    s->ws.d_result = (double *)((char *)blk + bp);
-    s->ws.d_counter = (unsigned int *)((char *)blk + bp + br);
+    s->ws.d_counter = (unsigned int *)((char *)blk + bp);
     PLK_CUDA(cudaMemsetAsync(s->ws.d_counter, 0, sizeof(unsigned int) * 4, s->stream));
     PLK_TRY(pinned_get(&s->ws.h_result));
+    s->ws.d_result = s->ws.h_result;
     return PLK_OK;
 }
 
