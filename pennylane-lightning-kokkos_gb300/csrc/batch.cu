@@ -29,6 +29,7 @@
 #include <string>
 #include <vector>
 
+#include "batch_tile.cuh"
 #include "window_host.cuh"
 
 namespace plk {
@@ -96,6 +97,7 @@ struct plk_batch_s {
     cudaGraphExec_t graph = nullptr;
     bool use_graph = true;
     int graph_cfg_key = -1;
+    plk::BatchTiles *tiles = nullptr; // complex64 without dense matrices: tile programs instead of the engine
     plk::LaunchPlan lp;      // launch plan of the configuration lp_key
     int lp_key = -1;
     float last_ms = 0.0f;
@@ -132,6 +134,8 @@ static void free_device(plk_batch b) {
         *p = nullptr;
     }
     b->scratch_bytes = 0;
+    if (b->tiles) batch_tiles_destroy(b->tiles);
+    b->tiles = nullptr;
     if (b->h_params_pinned) cudaFreeHost(b->h_params_pinned);
     if (b->h_out_pinned) cudaFreeHost(b->h_out_pinned);
     b->h_params_pinned = b->h_out_pinned = nullptr;
@@ -214,6 +218,19 @@ static int upload_vec(void **dptr, const void *src, size_t bytes, cudaStream_t s
     return PLK_OK;
 }
 
+// parameters and results, on the device and pinned
+static int alloc_io(plk_batch b) {
+    const size_t nc = b->circs.size(), np = std::max<size_t>(b->params.size(), 1);
+    PLK_CUDA(cudaMalloc(&b->d_params, np * sizeof(double)));
+    PLK_CUDA(cudaMemcpyAsync(b->d_params, b->params.data(), b->params.size() * sizeof(double), cudaMemcpyHostToDevice,
+                             b->stream));
+    PLK_CUDA(cudaMalloc(&b->d_expval, std::max<size_t>(nc, 1) * sizeof(double)));
+    PLK_CUDA(cudaMalloc(&b->d_jac, std::max(b->njac, 1) * sizeof(double)));
+    PLK_CUDA(cudaMallocHost(&b->h_params_pinned, np * sizeof(double)));
+    PLK_CUDA(cudaMallocHost(&b->h_out_pinned, (nc + b->njac + 1) * sizeof(double)));
+    return PLK_OK;
+}
+
 template <class T> static int upload_batch(plk_batch b) {
     using V = c2_t<T>;
     free_device(b);
@@ -235,16 +252,10 @@ template <class T> static int upload_batch(plk_batch b) {
                                  st));
     const size_t nc = b->circs.size();
     PLK_CUDA(cudaMalloc(&b->d_order, std::max<size_t>(nc, 1) * 2 * sizeof(int32_t)));
-    PLK_CUDA(cudaMalloc(&b->d_params, std::max<size_t>(b->params.size(), 1) * sizeof(double)));
-    PLK_CUDA(cudaMemcpyAsync(b->d_params, b->params.data(), b->params.size() * sizeof(double), cudaMemcpyHostToDevice,
-                             st));
-    PLK_CUDA(cudaMalloc(&b->d_expval, std::max<size_t>(nc, 1) * sizeof(double)));
-    PLK_CUDA(cudaMalloc(&b->d_jac, std::max(b->njac, 1) * sizeof(double)));
+    PLK_TRY(alloc_io(b));
     PLK_CUDA(cudaMalloc(&b->d_jac_part, std::max(b->njac, 1) * kMaxCluster * sizeof(double)));
     PLK_CUDA(cudaMalloc(&b->d_ev_part, std::max<size_t>(nc, 1) * kMaxCluster * sizeof(double)));
     PLK_CUDA(cudaMalloc(&b->d_counters, 4 * sizeof(unsigned)));
-    PLK_CUDA(cudaMallocHost(&b->h_params_pinned, std::max<size_t>(b->params.size(), 1) * sizeof(double)));
-    PLK_CUDA(cudaMallocHost(&b->h_out_pinned, (nc + b->njac + 1) * sizeof(double)));
     PLK_CUDA(cudaStreamSynchronize(st));
     return PLK_OK;
 }
@@ -579,9 +590,22 @@ static int cfg_key(const BatchConfig &c) {
 
 template <class T> static int prepare_run(plk_batch b) {
     if (!b->compiled) {
-        PLK_TRY(compile_batch(b));
-        PLK_TRY(upload_batch<T>(b));
+        if constexpr (sizeof(T) == 4) {
+            std::vector<BatchCircuit> circs;
+            for (const auto &c : b->circs) circs.push_back({c.nq, &c.ops, c.jac0, c.ntp, &c.terms});
+            free_device(b);
+            PLK_TRY(batch_tiles_create(circs, b->device, b->stream, &b->tiles));
+        }
+        if (b->tiles) {
+            PLK_TRY(alloc_io(b));
+            PLK_CUDA(cudaStreamSynchronize(b->stream));
+            b->compiled = true;
+        } else {
+            PLK_TRY(compile_batch(b));
+            PLK_TRY(upload_batch<T>(b));
+        }
     }
+    if (b->tiles) return PLK_OK;
     if (b->lp_key == cfg_key(b->cfg)) return PLK_OK;
     LaunchPlan &lp = b->lp;
     lp = LaunchPlan();
@@ -609,6 +633,7 @@ template <class T> static int prepare_run(plk_batch b) {
 
 // The stream work of one run: counters, matrices from parameters, engine.
 template <class T> static int enqueue_run(plk_batch b, const double *d_params, cudaStream_t st) {
+    if (b->tiles) return batch_tiles_enqueue(b->tiles, d_params, b->d_expval, b->d_jac, st);
     const LaunchPlan &lp = b->lp;
     PLK_CUDA(cudaMemsetAsync(b->d_counters, 0, 4 * sizeof(unsigned), st));
     const int np = (int)b->h_prep.size();
@@ -681,7 +706,7 @@ template <class T> static int run_host(plk_batch b, double *expval, double *jac)
     cudaEventElapsedTime(&b->last_ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    b->last_launches = b->h_prep.empty() ? 1 : 2;
+    b->last_launches = b->tiles ? batch_tiles_launches(b->tiles) : b->h_prep.empty() ? 1 : 2;
     if (expval) std::memcpy(expval, b->h_out_pinned, nc * sizeof(double));
     if (jac && b->njac) std::memcpy(jac, b->h_out_pinned + nc, b->njac * sizeof(double));
     return PLK_OK;

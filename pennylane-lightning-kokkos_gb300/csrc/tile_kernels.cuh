@@ -517,6 +517,11 @@ __device__ __forceinline__ AmpC128::V load_amp(const void *p, uint32_t i, int df
     const DF im = df_split_near(__longlong_as_double((long long)a.y));
     return {f2x_pack(re.hi, im.hi), f2x_pack(re.lo, im.lo)};
 }
+// amplitude i of |0...0>
+__device__ __forceinline__ f2x basis_amp(uint32_t i, f2x) { return f2x_pack(i == 0 ? 1.0f : 0.0f, 0.0f); }
+__device__ __forceinline__ AmpC128::V basis_amp(uint32_t i, AmpC128::V) {
+    return {f2x_pack(i == 0 ? 1.0f : 0.0f, 0.0f), 0ull};
+}
 __device__ __forceinline__ void store_amp(void *p, uint32_t i, int, f2x v) {
     __stcg(static_cast<unsigned long long *>(p) + i, v);
 }
@@ -528,10 +533,172 @@ __device__ __forceinline__ void store_amp(void *p, uint32_t i, int df, AmpC128::
     __stcg(static_cast<ulonglong2 *>(p) + i, make_ulonglong2(v.h, v.l));
 }
 
-template <class A, int R, bool BWD, int THREADS, int CTAS>
-__global__ void __launch_bounds__(THREADS, CTAS) k_tile(const __grid_constant__ Args a) {
+// A pass's blob in shared memory
+struct Pass {
+    const TileHdr &hd;
+    const TileRound *rounds;
+    const TileStage *stages;
+    const TileEvent *events;
+    const TileIndex *index;
+    const unsigned char *tab;
+    __device__ __forceinline__ explicit Pass(const unsigned char *p)
+        : hd(*reinterpret_cast<const TileHdr *>(p)),
+          rounds(reinterpret_cast<const TileRound *>(p + hd.off_rounds)),
+          stages(reinterpret_cast<const TileStage *>(p + hd.off_stages)),
+          events(reinterpret_cast<const TileEvent *>(p + hd.off_events)),
+          index(reinterpret_cast<const TileIndex *>(p + hd.off_index)), tab(p + hd.off_tab) {}
+};
+
+// state buffers of a sweep
+struct Buffers {
+    const void *lam_src;
+    void *lam, *hl;
+    int in_df, out_df; // complex128: double-float pairs on entry / exit
+    bool from_zero;    // the state is |0...0> on entry, lam_src is not read
+};
+
+// All rounds of one tile; every thread of the CTA takes part.  L, M: the tile's
+// slots of lambda and H lambda; row: this warp's accumulators.
+template <class A, int R, bool BWD>
+__device__ __forceinline__ void run_tile(const Pass &ps, const Buffers &bf, int tile, int T, unsigned char *L,
+                                         unsigned char *M, float2 *row) {
     using V = typename A::V;
     constexpr int NA = 1 << R;
+    const TileHdr &hd = ps.hd;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nrounds = hd.nrounds;
+    uint32_t base = (uint32_t)tile;
+    for (int k = 0; k < T; k++) {
+        const uint32_t lo = base & ((1u << hd.gpos[k]) - 1u);
+        base = ((base ^ lo) << 1) | lo;
+    }
+    uint32_t ev = 0;
+    for (int r = 0; r < nrounds; r++) {
+        const TileRound &q = ps.rounds[r];
+        uint32_t gev = base;
+        for (int k = 0; k < q.nev; k++)
+            if (base >> ps.events[q.ev0 + k].bit & 1u) {
+                ev ^= ps.events[q.ev0 + k].mask;
+                gev ^= ps.events[q.ev0 + k].gmask;
+            }
+        const uint32_t o = q.lo[lane] ^ q.hi[warp] ^ q.xorc ^ ev;
+        const uint32_t r0 = q.rcol[0], r1 = q.rcol[1], r2 = q.rcol[2], r3 = q.rcol[3];
+        const uint32_t r01 = r0 ^ r1, r23 = r2 ^ r3; // one three-input operation per slot
+        auto slot = [&](int j) {
+            return o ^ ((j & 3) == 3 ? r01 : (j & 1) ? r0 : (j & 2) ? r1 : 0u) ^
+                   ((j & 12) == 12 ? r23 : (j & 4) ? r2 : (j & 8) ? r3 : 0u);
+        };
+        V v[NA], h[NA];
+        if (r == 0) {
+            const TileIndex &x = ps.index[hd.load_idx];
+            const uint32_t g = gev ^ x.lo[lane] ^ x.hi[warp] ^ x.c;
+            const uint32_t g0 = x.r[0], g1 = x.r[1], g2 = x.r[2], g3 = x.r[3], g01 = g0 ^ g1, g23 = g2 ^ g3;
+            const void *lam = bf.lam_src, *hl = bf.hl;
+#pragma unroll
+            for (int j = 0; j < NA; j++) {
+                const uint32_t i = g ^ ((j & 3) == 3 ? g01 : (j & 1) ? g0 : (j & 2) ? g1 : 0u) ^
+                                   ((j & 12) == 12 ? g23 : (j & 4) ? g2 : (j & 8) ? g3 : 0u);
+                v[j] = bf.from_zero ? basis_amp(i, V{}) : load_amp(lam, i, bf.in_df, V{});
+                if (BWD) h[j] = load_amp(hl, i, bf.in_df, V{});
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < NA; j++) {
+                v[j] = A::ld(L + slot(j));
+                if (BWD) h[j] = A::ld(M + slot(j));
+            }
+        }
+        uint32_t gi = base;
+        if (q.idx != 0xffffu) gi |= ps.index[q.idx].lo[lane] | ps.index[q.idx].hi[warp];
+        for (int k = 0; k < q.nstages; k++) {
+            const TileStage &st = ps.stages[q.stage0 + k];
+            DF y[8] = {}; // Y sums by bit, then Z sums by bit
+            DF x[4] = {};
+            bool zbits = false;
+            if (BWD && (st.table & 1)) {
+                zbits = (st.zsel & ~0x0116u) == 0;
+                if (zbits) walsh_bits<A, R>(v, h, y + 4);
+                else walsh_all<A, R>(v, h, st.zsel, st.acc_z, row, lane);
+            }
+            if (st.table & 2) {
+                const auto *e = reinterpret_cast<const typename Form<A>::E *>(ps.tab) + st.tab;
+#pragma unroll
+                for (int j = 0; j < NA; j++) {
+                    const auto z = e[j];
+                    phase(v[j], z);
+                    if (BWD) phase(h[j], z);
+                }
+            }
+            {
+                DF(&y4)[4] = reinterpret_cast<DF(&)[4]>(y);
+                step_ry<A, R, BWD, 0>(v, h, st, y4, x);
+                step_ry<A, R, BWD, 1>(v, h, st, y4, x);
+                step_ry<A, R, BWD, 2>(v, h, st, y4, x);
+                step_ry<A, R, BWD, 3>(v, h, st, y4, x);
+            }
+            if (BWD) {
+                if (zbits || (st.sums & 1)) {
+                    int id[8], next = st.acc_z;
+#pragma unroll
+                    for (int b = 0; b < 4; b++) {
+                        id[b] = (st.ry >> b & 1) ? st.acc_y[b] : -1;
+                        id[4 + b] = (zbits && (st.zsel >> (1 << b) & 1)) ? next++ : -1;
+                    }
+                    warp_sums<8>(y, id, row, lane);
+                }
+                if (st.sums & 2) {
+                    int id[4];
+#pragma unroll
+                    for (int b = 0; b < 4; b++) id[b] = (st.ry >> b & 1) ? st.acc_x[b] : -1;
+                    warp_sums<4>(x, id, row, lane);
+                }
+            }
+            if (st.special == TS_CRY) {
+                const uint32_t act = (gi & st.cmask) == st.cval ? st.jact : 0u;
+                DF c = {0.0f, 0.0f};
+                switch (st.bit) {
+                case 0: step_cry<A, R, BWD, 0>(v, h, st, act, c); break;
+                case 1: step_cry<A, R, BWD, 1>(v, h, st, act, c); break;
+                case 2: step_cry<A, R, BWD, 2>(v, h, st, act, c); break;
+                default: step_cry<A, R, BWD, 3>(v, h, st, act, c); break;
+                }
+                if (BWD && st.sacc >= 0) {
+                    c = warp_sum(c);
+                    if (lane == 0) acc_add(row, st.sacc, c);
+                }
+            } else if (st.special != TS_NONE) {
+                step_index<A, R, BWD>(v, h, st, ps.index[q.idx], gi, ps.tab, row, lane);
+            }
+        }
+        if (r + 1 < nrounds) {
+#pragma unroll
+            for (int j = 0; j < NA; j++) {
+                A::st(L + slot(j), v[j]);
+                if (BWD) A::st(M + slot(j), h[j]);
+            }
+        } else {
+            if (nrounds == 1) __syncthreads(); // all of the tile read before any of it is written
+            uint32_t go = base;
+            for (int k = hd.ev_store0; k < hd.nev; k++)
+                if (base >> ps.events[k].bit & 1u) go ^= ps.events[k].gmask;
+            const TileIndex &x = ps.index[hd.store_idx];
+            const uint32_t g = go ^ x.lo[lane] ^ x.hi[warp] ^ x.c;
+            const uint32_t g0 = x.r[0], g1 = x.r[1], g2 = x.r[2], g3 = x.r[3], g01 = g0 ^ g1, g23 = g2 ^ g3;
+            void *lam = bf.lam, *hl = bf.hl;
+#pragma unroll
+            for (int j = 0; j < NA; j++) {
+                const uint32_t i = g ^ ((j & 3) == 3 ? g01 : (j & 1) ? g0 : (j & 2) ? g1 : 0u) ^
+                                   ((j & 12) == 12 ? g23 : (j & 4) ? g2 : (j & 8) ? g3 : 0u);
+                store_amp(lam, i, bf.out_df, v[j]);
+                if (BWD) store_amp(hl, i, bf.out_df, h[j]);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+template <class A, int R, bool BWD, int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS) k_tile(const __grid_constant__ Args a) {
     extern __shared__ __align__(16) unsigned char tile_smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t tile_bytes = (uint32_t)A::kBytes << a.T;
@@ -544,148 +711,14 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_tile(const __grid_constant__ 
     if (BWD)
         for (int i = lane; i < a.nacc; i += 32) row[i] = make_float2(0.0f, 0.0f);
     __syncthreads();
-    const TileHdr &hd = *reinterpret_cast<const TileHdr *>(prog);
-    const TileRound *rounds = reinterpret_cast<const TileRound *>(prog + hd.off_rounds);
-    const TileStage *stages = reinterpret_cast<const TileStage *>(prog + hd.off_stages);
-    const TileEvent *events = reinterpret_cast<const TileEvent *>(prog + hd.off_events);
-    const TileIndex *index = reinterpret_cast<const TileIndex *>(prog + hd.off_index);
-    const unsigned char *tab = prog + hd.off_tab;
-    const int nrounds = hd.nrounds;
-    for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
-        uint32_t base = (uint32_t)tile;
-        for (int k = 0; k < a.T; k++) {
-            const uint32_t lo = base & ((1u << hd.gpos[k]) - 1u);
-            base = ((base ^ lo) << 1) | lo;
-        }
-        uint32_t ev = 0;
-        for (int r = 0; r < nrounds; r++) {
-            const TileRound &q = rounds[r];
-            uint32_t gev = base;
-            for (int k = 0; k < q.nev; k++)
-                if (base >> events[q.ev0 + k].bit & 1u) {
-                    ev ^= events[q.ev0 + k].mask;
-                    gev ^= events[q.ev0 + k].gmask;
-                }
-            const uint32_t o = q.lo[lane] ^ q.hi[warp] ^ q.xorc ^ ev;
-            const uint32_t r0 = q.rcol[0], r1 = q.rcol[1], r2 = q.rcol[2], r3 = q.rcol[3];
-            const uint32_t r01 = r0 ^ r1, r23 = r2 ^ r3; // one three-input operation per slot
-            auto slot = [&](int j) {
-                return o ^ ((j & 3) == 3 ? r01 : (j & 1) ? r0 : (j & 2) ? r1 : 0u) ^
-                       ((j & 12) == 12 ? r23 : (j & 4) ? r2 : (j & 8) ? r3 : 0u);
-            };
-            V v[NA], h[NA];
-            if (r == 0) {
-                const TileIndex &x = index[hd.load_idx];
-                const uint32_t g = gev ^ x.lo[lane] ^ x.hi[warp] ^ x.c;
-                const uint32_t g0 = x.r[0], g1 = x.r[1], g2 = x.r[2], g3 = x.r[3], g01 = g0 ^ g1, g23 = g2 ^ g3;
-                const void *lam = a.lam_src[blockIdx.y], *hl = a.hl[blockIdx.y];
-#pragma unroll
-                for (int j = 0; j < NA; j++) {
-                    const uint32_t i = g ^ ((j & 3) == 3 ? g01 : (j & 1) ? g0 : (j & 2) ? g1 : 0u) ^
-                                       ((j & 12) == 12 ? g23 : (j & 4) ? g2 : (j & 8) ? g3 : 0u);
-                    v[j] = load_amp(lam, i, a.in_df, V{});
-                    if (BWD) h[j] = load_amp(hl, i, a.in_df, V{});
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < NA; j++) {
-                    v[j] = A::ld(L + slot(j));
-                    if (BWD) h[j] = A::ld(M + slot(j));
-                }
-            }
-            uint32_t gi = base;
-            if (q.idx != 0xffffu) gi |= index[q.idx].lo[lane] | index[q.idx].hi[warp];
-            for (int k = 0; k < q.nstages; k++) {
-                const TileStage &st = stages[q.stage0 + k];
-                DF y[8] = {}; // Y sums by bit, then Z sums by bit
-                DF x[4] = {};
-                bool zbits = false;
-                if (BWD && (st.table & 1)) {
-                    zbits = (st.zsel & ~0x0116u) == 0;
-                    if (zbits) walsh_bits<A, R>(v, h, y + 4);
-                    else walsh_all<A, R>(v, h, st.zsel, st.acc_z, row, lane);
-                }
-                if (st.table & 2) {
-                    const auto *e = reinterpret_cast<const typename Form<A>::E *>(tab) + st.tab;
-#pragma unroll
-                    for (int j = 0; j < NA; j++) {
-                        const auto z = e[j];
-                        phase(v[j], z);
-                        if (BWD) phase(h[j], z);
-                    }
-                }
-                {
-                    DF(&y4)[4] = reinterpret_cast<DF(&)[4]>(y);
-                    step_ry<A, R, BWD, 0>(v, h, st, y4, x);
-                    step_ry<A, R, BWD, 1>(v, h, st, y4, x);
-                    step_ry<A, R, BWD, 2>(v, h, st, y4, x);
-                    step_ry<A, R, BWD, 3>(v, h, st, y4, x);
-                }
-                if (BWD) {
-                    if (zbits || (st.sums & 1)) {
-                        int id[8], next = st.acc_z;
-#pragma unroll
-                        for (int b = 0; b < 4; b++) {
-                            id[b] = (st.ry >> b & 1) ? st.acc_y[b] : -1;
-                            id[4 + b] = (zbits && (st.zsel >> (1 << b) & 1)) ? next++ : -1;
-                        }
-                        warp_sums<8>(y, id, row, lane);
-                    }
-                    if (st.sums & 2) {
-                        int id[4];
-#pragma unroll
-                        for (int b = 0; b < 4; b++) id[b] = (st.ry >> b & 1) ? st.acc_x[b] : -1;
-                        warp_sums<4>(x, id, row, lane);
-                    }
-                }
-                if (st.special == TS_CRY) {
-                    const uint32_t act = (gi & st.cmask) == st.cval ? st.jact : 0u;
-                    DF c = {0.0f, 0.0f};
-                    switch (st.bit) {
-                    case 0: step_cry<A, R, BWD, 0>(v, h, st, act, c); break;
-                    case 1: step_cry<A, R, BWD, 1>(v, h, st, act, c); break;
-                    case 2: step_cry<A, R, BWD, 2>(v, h, st, act, c); break;
-                    default: step_cry<A, R, BWD, 3>(v, h, st, act, c); break;
-                    }
-                    if (BWD && st.sacc >= 0) {
-                        c = warp_sum(c);
-                        if (lane == 0) acc_add(row, st.sacc, c);
-                    }
-                } else if (st.special != TS_NONE) {
-                    step_index<A, R, BWD>(v, h, st, index[q.idx], gi, tab, row, lane);
-                }
-            }
-            if (r + 1 < nrounds) {
-#pragma unroll
-                for (int j = 0; j < NA; j++) {
-                    A::st(L + slot(j), v[j]);
-                    if (BWD) A::st(M + slot(j), h[j]);
-                }
-            } else {
-                if (nrounds == 1) __syncthreads(); // all of the tile read before any of it is written
-                uint32_t go = base;
-                for (int k = hd.ev_store0; k < hd.nev; k++)
-                    if (base >> events[k].bit & 1u) go ^= events[k].gmask;
-                const TileIndex &x = index[hd.store_idx];
-                const uint32_t g = go ^ x.lo[lane] ^ x.hi[warp] ^ x.c;
-                const uint32_t g0 = x.r[0], g1 = x.r[1], g2 = x.r[2], g3 = x.r[3], g01 = g0 ^ g1, g23 = g2 ^ g3;
-                void *lam = a.lam[blockIdx.y], *hl = a.hl[blockIdx.y];
-#pragma unroll
-                for (int j = 0; j < NA; j++) {
-                    const uint32_t i = g ^ ((j & 3) == 3 ? g01 : (j & 1) ? g0 : (j & 2) ? g1 : 0u) ^
-                                       ((j & 12) == 12 ? g23 : (j & 4) ? g2 : (j & 8) ? g3 : 0u);
-                    store_amp(lam, i, a.out_df, v[j]);
-                    if (BWD) store_amp(hl, i, a.out_df, h[j]);
-                }
-            }
-            __syncthreads();
-        }
-    }
+    const Pass ps(prog);
+    const Buffers bf{a.lam_src[blockIdx.y], a.lam[blockIdx.y], a.hl[blockIdx.y], a.in_df, a.out_df, false};
+    for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) run_tile<A, R, BWD>(ps, bf, tile, a.T, L, M, row);
     if (BWD) {
         for (int i = tid; i < a.nacc; i += blockDim.x) {
             DF t = {0.0f, 0.0f};
             for (int w = 0; w < (int)blockDim.x / 32; w++) df_add(acc[w * a.nacc + i].x, acc[w * a.nacc + i].y, t.hi, t.lo);
-            a.part[((size_t)blockIdx.y * a.nacc_all + hd.acc0 + i) * gridDim.x + blockIdx.x] = df_result(t.hi, t.lo);
+            a.part[((size_t)blockIdx.y * a.nacc_all + ps.hd.acc0 + i) * gridDim.x + blockIdx.x] = df_result(t.hi, t.lo);
         }
     }
 }

@@ -37,6 +37,7 @@
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <map>
@@ -123,6 +124,7 @@ struct TilePass {
 struct JacTerm {
     int32_t slot, acc;
     double coef;
+    int32_t ref = -1; // symbolic programs: the coefficient is coef * refs[ref]
 };
 
 struct TileProgram {
@@ -199,8 +201,59 @@ struct Grad {
 
 enum PrimKind { P_U1, P_DIAG, P_PAR, P_CRY, P_CX, P_X, P_SWAP };
 
+// ---- symbolic programs -----------------------------------------------------
+// A batch compiles its circuits once, for any parameters: the program's numbers
+// (tables, rotations, coefficients) are left open and listed here, and a kernel
+// fills them in for each run (batch_tile.cu).  A gate's entries are
+// A0 + A1 cos(t/2) + A2 sin(t/2) + A3 cos(t) + A4 sin(t): `basis` is the offset
+// of its five coefficients per entry.
+enum GateForm : uint8_t { GF_DIAG = 0, GF_RY = 1, GF_OTHER = 2 };
+enum RunType : uint8_t { RT_DIAG = 0, RT_RIGHT = 1, RT_LEFT = 2, RT_GENERAL = 3 };
+
+struct SymGate { // one gate of a run of one-wire gates
+    int32_t basis, pidx; // pidx -1: constant
+    int32_t next;        // the run's next gate, -1 at its end
+    int32_t form;
+    double g[4];         // generator: coefficients of I, X, Y, Z
+    int32_t ref[4];      // refs of its I, X, Y, Z coefficients in the frame of the run's sums (-1: not wanted)
+};
+struct SymRun { // diag(b) RY(c, s) diag(a), or the diagonal itself
+    int32_t head, type;
+    int32_t pool_a, pool_b; // two entries each; RT_DIAG: pool_a
+};
+struct SymEval { // entries of another gate
+    int32_t basis, pidx, n, pool;
+};
+struct SymFactor { // part of a table: pool[k], k = register bits reg[0..K) of j; K = -1: the parity of j & mask
+    int32_t pool;
+    int8_t K;
+    uint8_t reg[3];
+    uint8_t mask, pad[3];
+};
+struct SymTable { // a phase table: the product of its factors
+    int32_t pass;
+    uint32_t off; // byte offset in the pass's blob
+    int32_t first, count;
+};
+struct SymPatch { // kind 0: rotation of run `src`; 1: c, s from pool; 2: n entries from pool
+    int32_t pass;
+    uint32_t off;
+    int32_t kind, src, n;
+};
+struct Symbols {
+    std::vector<SymGate> gates;
+    std::vector<SymRun> runs;
+    std::vector<SymEval> evals;
+    std::vector<SymFactor> factors;
+    std::vector<SymTable> tables;
+    std::vector<SymPatch> patches;
+    int npool = 0, nrefs = 0;
+};
+
 struct Prim {
     int kind = P_U1;
+    int sbasis = -1, spidx = -1;      // symbolic: coefficients of the entries
+    int shead = -1, stail = -1;       // symbolic U1: its gates
     int t = 0, t2 = 0;          // target state bits
     uint32_t cmask = 0, cval = 0; // CRY controls; CX: control bit mask
     double c = 1, s = 0;        // CRY
@@ -474,10 +527,14 @@ inline void invert(std::vector<Prim> &v) {
 // is accessed as D by both (block diagonal in it) or as F by both (flips).
 enum Access : uint8_t { AC_N = 0, AC_D = 1, AC_F = 2 };
 
-struct ZTerm { // coef * (Walsh sum of the state bits in mask) enters Jacobian slot
-    uint32_t mask;
+struct Term { // coef * (a sum) enters Jacobian slot
     int slot;
     double coef;
+    int ref = -1;
+};
+struct ZTerm : Term { // the Walsh sum of the state bits in mask
+    uint32_t mask;
+    ZTerm(uint32_t m, int s, double c, int r = -1) : Term{s, c, r}, mask(m) {}
 };
 
 struct Unit {
@@ -486,8 +543,9 @@ struct Unit {
     cplx a0 = 1, a1 = 1, b0 = 1, b1 = 1; // U1: diag(b) RY(c, s) diag(a), |s| <= c
     bool has_a = false, has_b = false;
     // gradient terms (Jacobian slot, coefficient)
-    std::vector<std::pair<int, double>> gx, gy; // U1, CRY
-    std::vector<ZTerm> gz;                      // U1, DIAG, PAR
+    std::vector<Term> gx, gy; // U1, CRY
+    std::vector<ZTerm> gz;    // U1, DIAG, PAR
+    int srun = -1, pool_a = -1, pool_b = -1; // symbolic: run, entries of a (diagonals: the entries) and b
     uint32_t bits = 0; // all state bits touched
     uint32_t need = 0; // bits that have to be in the tile
     uint32_t reg = 0;  // bits that have to be register bits
@@ -504,7 +562,7 @@ struct Options {
 
 class Compiler {
   public:
-    Compiler(int nq, bool bwd, const Options &o) : nq_(nq), bwd_(bwd), o_(o) {
+    Compiler(int nq, bool bwd, const Options &o, Symbols *sym = nullptr) : nq_(nq), bwd_(bwd), o_(o), sym_(sym) {
         T_ = std::min(o.T, nq);
         R_ = std::min(o.R, T_);
         last_.assign(nq, -1);
@@ -541,8 +599,15 @@ class Compiler {
             int nacc = 0;
             const double pend = pend_;
             const Table last_table = last_table_;
+            const size_t nf = sym_ ? sym_->factors.size() : 0, nt = sym_ ? sym_->tables.size() : 0;
+            const size_t np = sym_ ? sym_->patches.size() : 0;
             for (;;) {
                 jac.clear();
+                if (sym_) {
+                    sym_->factors.resize(nf);
+                    sym_->tables.resize(nt);
+                    sym_->patches.resize(np);
+                }
                 pend_ = pend;
                 last_table_ = last_table;
                 pass_ = (int)P.passes.size();
@@ -582,6 +647,7 @@ class Compiler {
     int nq_, T_ = 0, R_ = 0;
     bool bwd_;
     Options o_;
+    Symbols *sym_ = nullptr;
     std::vector<Prim> prims_;
     std::vector<int> last_; // last primitive touching each bit
     std::vector<Unit> units_;
@@ -622,13 +688,100 @@ class Compiler {
     void add_prim(const Prim &p) {
         if (p.kind == P_U1) {
             const int l = last_[p.t];
+            const int g = sym_ ? add_gate(p) : -1;
             if (l >= 0 && prims_[l].kind == P_U1) {
-                merge_u1(prims_[l], p);
+                if (sym_) {
+                    sym_->gates[prims_[l].stail].next = g;
+                    prims_[l].stail = g;
+                    prims_[l].grads.insert(prims_[l].grads.end(), p.grads.begin(), p.grads.end());
+                } else {
+                    merge_u1(prims_[l], p);
+                }
                 return;
             }
+            last_[p.t] = (int)prims_.size();
+            prims_.push_back(p);
+            prims_.back().shead = prims_.back().stail = g;
+            return;
         }
         for (uint32_t m = bits_of(p); m; m &= m - 1) last_[__builtin_ctz(m)] = (int)prims_.size();
         prims_.push_back(p);
+    }
+
+    int add_gate(const Prim &p) {
+        SymGate g;
+        g.basis = p.sbasis;
+        g.pidx = p.spidx;
+        g.next = -1;
+        // the form at the sample parameters of p is the form at all of them
+        const bool diag = p.m[1] == 0.0 && p.m[2] == 0.0;
+        const bool ry = !diag && p.m[0] == p.m[3] && p.m[1] == -p.m[2] && p.m[0].imag() == 0.0 && p.m[1].imag() == 0.0;
+        g.form = diag ? GF_DIAG : ry ? GF_RY : GF_OTHER;
+        for (int k = 0; k < 4; k++) {
+            g.g[k] = p.grads.empty() ? 0.0 : p.grads[0].g[k];
+            g.ref[k] = -1;
+        }
+        sym_->gates.push_back(g);
+        return (int)sym_->gates.size() - 1;
+    }
+
+    // A run's type and the sums that its generators need, from the forms alone.
+    void symbolic_run(Unit &u, Prim &p) {
+        int first = -1, last = -1, n = 0, others = 0, diag_inside = 0;
+        for (int g = p.shead; g >= 0; g = sym_->gates[g].next, n++)
+            if (sym_->gates[g].form != GF_DIAG) {
+                if (first < 0) first = n;
+                last = n;
+                others += sym_->gates[g].form == GF_OTHER;
+            }
+        n = 0;
+        for (int g = p.shead; g >= 0; g = sym_->gates[g].next, n++)
+            diag_inside += n > first && n < last && sym_->gates[g].form == GF_DIAG;
+        SymRun r;
+        r.head = p.shead;
+        r.type = first < 0 ? RT_DIAG
+                 : others || diag_inside || (first > 0 && last + 1 < n) ? RT_GENERAL
+                 : last + 1 < n ? RT_LEFT
+                                : RT_RIGHT;
+        r.pool_a = r.pool_b = -1;
+        if (r.type != RT_LEFT) {
+            r.pool_a = sym_->npool;
+            sym_->npool += 2;
+        }
+        if (r.type == RT_LEFT || r.type == RT_GENERAL) {
+            r.pool_b = sym_->npool;
+            sym_->npool += 2;
+        }
+        const uint32_t b = 1u << p.t;
+        size_t grad = 0;
+        int k = 0;
+        for (int gi = p.shead; gi >= 0; gi = sym_->gates[gi].next, k++) {
+            SymGate &g = sym_->gates[gi];
+            if (g.g[0] == 0 && g.g[1] == 0 && g.g[2] == 0 && g.g[3] == 0) continue;
+            const int slot = p.grads[grad++].slot;
+            const bool start = first < 0 || k <= first; // only diagonals before it
+            const bool plain = start && g.form == GF_DIAG;
+            const bool only_y = g.form == GF_RY && r.type != RT_GENERAL;
+            auto ref = [&](int c) { return g.ref[c] = sym_->nrefs++; };
+            if (g.g[0] != 0) u.gz.push_back(ZTerm(0, slot, 1.0, ref(0)));
+            if (!only_y) u.gz.push_back(ZTerm(b, slot, 1.0, ref(3)));
+            if (!plain) {
+                u.gy.push_back(Term{slot, 1.0, ref(2)});
+                if (!only_y) u.gx.push_back(Term{slot, 1.0, ref(1)});
+            }
+        }
+        u.srun = (int)sym_->runs.size();
+        u.pool_a = r.pool_a;
+        u.pool_b = r.pool_b;
+        u.has_a = r.type == RT_RIGHT || r.type == RT_GENERAL;
+        u.has_b = r.pool_b >= 0;
+        if (r.type == RT_DIAG) {
+            u.kind = p.kind = P_DIAG;
+            p.K = 1;
+            p.db[0] = p.t;
+        }
+        sym_->runs.push_back(r);
+        u.p = std::move(p);
     }
 
     // a <- p a; p's generators (before p acts) in the frame of a's start
@@ -701,7 +854,7 @@ class Compiler {
     }
 
     static void add_gz(Unit &u, uint32_t mask, int slot, double coef) {
-        if (std::fabs(coef) >= kTiny) u.gz.push_back(ZTerm{mask, slot, coef});
+        if (std::fabs(coef) >= kTiny) u.gz.push_back(ZTerm(mask, slot, coef));
     }
 
     void make_units() {
@@ -712,7 +865,15 @@ class Compiler {
             u.kind = p.kind;
             u.bits = bits_of(p);
             bool flip = false;
-            if (p.kind == P_U1) {
+            if (sym_ && (p.kind == P_DIAG || p.kind == P_PAR || p.kind == P_CRY)) {
+                const int n = p.kind == P_DIAG ? 1 << p.K : 2;
+                u.pool_a = sym_->npool;
+                sym_->npool += n;
+                sym_->evals.push_back(SymEval{p.sbasis, p.spidx, n, u.pool_a});
+            }
+            if (p.kind == P_U1 && sym_) {
+                symbolic_run(u, p);
+            } else if (p.kind == P_U1) {
                 const uint32_t b = 1u << p.t;
                 if (std::norm(p.m[2]) > std::norm(p.m[0])) { // take an X out on the left
                     flip = true;
@@ -762,7 +923,7 @@ class Compiler {
                 }
             } else {
                 if (p.kind == P_CRY) {
-                    for (const Grad &e : p.grads) u.gy.push_back({e.slot, e.g[2]});
+                    for (const Grad &e : p.grads) u.gy.push_back(Term{e.slot, e.g[2]});
                 } else if (p.kind == P_PAR) {
                     for (const Grad &e : p.grads) add_gz(u, p.pmask, e.slot, e.g[3]);
                 } else if (p.kind == P_DIAG) {
@@ -828,8 +989,8 @@ class Compiler {
         for (const Grad &e : p.grads) {
             const double gx = e.g[1] * ph.real() - e.g[2] * ph.imag();
             const double gy = e.g[1] * ph.imag() + e.g[2] * ph.real();
-            if (std::fabs(gx) >= kTiny) u.gx.push_back({e.slot, gx});
-            if (std::fabs(gy) >= kTiny) u.gy.push_back({e.slot, gy});
+            if (std::fabs(gx) >= kTiny) u.gx.push_back(Term{e.slot, gx});
+            if (std::fabs(gy) >= kTiny) u.gy.push_back(Term{e.slot, gy});
             add_gz(u, 0, e.slot, e.g[0]);
             add_gz(u, b, e.slot, e.g[3]);
         }
@@ -930,12 +1091,13 @@ class Compiler {
     }
 
     // -------------------------------------------------------------- passes --
-    using Terms = std::vector<std::pair<int, double>>; // (Jacobian slot, coefficient)
+    using Terms = std::vector<Term>;
 
     struct Factor { // a diagonal factor of a table: a unit's, or one side of a run
         const Unit *u = nullptr;
         int bit = 0;
         cplx e0 = 1, e1 = 1;
+        int pool = -1;
     };
     enum StepKind { SK_RY, SK_CRY, SK_TAB, SK_INDEX };
     struct Step {
@@ -979,14 +1141,14 @@ class Compiler {
             const uint32_t b = 1u << u.p.t;
             if (u.has_a || !u.gz.empty()) {
                 Step &t = table_for(st, b, false);
-                if (u.has_a) t.f.push_back(Factor{nullptr, u.p.t, u.a0, u.a1});
+                if (u.has_a) t.f.push_back(Factor{nullptr, u.p.t, u.a0, u.a1, u.pool_a});
                 t.gz.insert(t.gz.end(), u.gz.begin(), u.gz.end());
             }
             place_turn(st, u);
-            if (u.has_b) table_for(st, b, true).f.push_back(Factor{nullptr, u.p.t, u.b0, u.b1});
+            if (u.has_b) table_for(st, b, true).f.push_back(Factor{nullptr, u.p.t, u.b0, u.b1, u.pool_b});
         } else if ((u.bits & ~regs) == 0) {
             Step &t = table_for(st, u.bits, false);
-            t.f.push_back(Factor{&u, 0, 1, 1});
+            t.f.push_back(Factor{&u, 0, 1, 1, u.pool_a});
             t.gz.insert(t.gz.end(), u.gz.begin(), u.gz.end());
         } else {
             Step d;
@@ -1158,7 +1320,7 @@ class Compiler {
         bool want_index = false;
         auto acc = [&](const Terms &t) -> int16_t {
             if (t.empty()) return -1;
-            for (const auto &e : t) jac.push_back(JacTerm{e.first, acc0 + nacc, e.second * pend_ * pend_});
+            for (const Term &e : t) jac.push_back(JacTerm{e.slot, acc0 + nacc, e.coef * pend_ * pend_, e.ref});
             return (int16_t)nacc++;
         };
         auto reg_of = [&](int state_bit) {
@@ -1189,6 +1351,10 @@ class Compiler {
                 if (!turn[b]) continue;
                 const Unit &u = *turn[b];
                 cur.ry |= (uint8_t)(1u << b);
+                if (sym_)
+                    sym_->patches.push_back(SymPatch{
+                        pass_, (uint32_t)(o.stages.size() * sizeof(TileStage) + offsetof(TileStage, rot) + 16 * b), 0,
+                        u.srun, 0});
                 if (scaled()) {
                     put2(cur.rot[b], u.p.s / u.p.c);
                 } else {
@@ -1220,6 +1386,26 @@ class Compiler {
                     cplx e[kMaxAmps];
                     for (int j = 0; j < amps; j++) e[j] = pend_;
                     pend_ = 1;
+                    if (sym_) {
+                        sym_->tables.push_back(SymTable{pass_, (uint32_t)(cur.tab * o_.amp_bytes),
+                                                        (int32_t)sym_->factors.size(), (int32_t)s.f.size()});
+                        for (const Factor &f : s.f) {
+                            SymFactor q;
+                            std::memset(&q, 0, sizeof(q));
+                            q.pool = f.pool;
+                            if (!f.u) {
+                                q.K = 1;
+                                q.reg[0] = (uint8_t)reg_of(f.bit);
+                            } else if (f.u->kind == P_PAR) {
+                                q.K = -1;
+                                q.mask = (uint8_t)reg_mask(f.u->p.pmask);
+                            } else {
+                                q.K = (int8_t)f.u->p.K;
+                                for (int i = 0; i < f.u->p.K; i++) q.reg[i] = (uint8_t)reg_of(f.u->p.db[i]);
+                            }
+                            sym_->factors.push_back(q);
+                        }
+                    }
                     for (const Factor &f : s.f) {
                         if (!f.u) {
                             const int i = reg_of(f.bit);
@@ -1250,7 +1436,7 @@ class Compiler {
                             cur.zsel |= (uint16_t)(1u << z[i].first);
                             nacc++;
                         }
-                        jac.push_back(JacTerm{z[i].second->slot, acc0 + nacc - 1, z[i].second->coef * scale * scale});
+                        jac.push_back(JacTerm{z[i].second->slot, acc0 + nacc - 1, z[i].second->coef * scale * scale, z[i].second->ref});
                     }
                 }
                 if (cur.table & 2) last_table_ = Table{pass_, cur.tab, jac0_ + jac.size()};
@@ -1273,19 +1459,26 @@ class Compiler {
                     cur.cmask = u.p.cmask & ~regs;
                     cur.cval = u.p.cval & ~regs;
                     want_index = want_index || cur.cmask != 0;
+                    if (sym_)
+                        sym_->patches.push_back(SymPatch{
+                            pass_, (uint32_t)(o.stages.size() * sizeof(TileStage) + offsetof(TileStage, coef)), 1, u.pool_a,
+                            2});
                     put2(cur.coef, u.p.c);
                     put2(cur.coef + 2, u.p.s);
                     cur.sacc = acc(u.gy);
                 } else {
                     want_index = true;
                     cur.stab = (uint16_t)tab_pos(o);
+                    if (sym_)
+                        sym_->patches.push_back(SymPatch{pass_, (uint32_t)(cur.stab * o_.amp_bytes), 2, u.pool_a,
+                                                         u.kind == P_PAR ? 2 : 1 << u.p.K});
                     if (u.kind == P_PAR) {
                         cur.special = TS_PAR;
                         cur.cmask = u.p.pmask;
                         put(o, u.p.d[0]);
                         put(o, u.p.d[1]);
                         Terms g;
-                        for (const ZTerm &e : u.gz) g.push_back({e.slot, e.coef});
+                        for (const ZTerm &e : u.gz) g.push_back(Term{e.slot, e.coef, e.ref});
                         cur.sacc = acc(g);
                     } else {
                         cur.special = TS_DIAG;
@@ -1296,7 +1489,7 @@ class Compiler {
                         for (const Grad &e : u.p.grads) {
                             cur.gtab = (uint32_t)o.tab.size();
                             for (double x : e.table) o.tab.push_back((float)x);
-                            cur.sacc = acc(Terms{{e.slot, e.coef}});
+                            cur.sacc = acc(Terms{Term{e.slot, e.coef}});
                         }
                         while (o.tab.size() % (o_.amp_bytes / sizeof(float))) o.tab.push_back(0.0f);
                     }
@@ -1455,6 +1648,11 @@ class Compiler {
         h.off_index = area(o.index.size() * sizeof(TileIndex));
         h.off_tab = area(o.tab.size() * sizeof(float));
         h.bytes = (uint32_t)at;
+        if (sym_) { // offsets within the blob
+            for (size_t i = sym_->tables.size(); i-- > 0 && sym_->tables[i].pass == pass_;) sym_->tables[i].off += h.off_tab;
+            for (size_t i = sym_->patches.size(); i-- > 0 && sym_->patches[i].pass == pass_;)
+                sym_->patches[i].off += sym_->patches[i].kind == 2 ? h.off_tab : h.off_stages;
+        }
         pass.blob.assign(at, 0);
         auto cp = [&](uint32_t off, const void *src, size_t bytes) {
             if (bytes) std::memcpy(pass.blob.data() + off, src, bytes);
