@@ -109,18 +109,33 @@ class AdjointCircuit:
             self.ops.append((g, wires, inv, k if npar == 1 else -1))
             k += npar
         self.num_params = k
-        self._wire_arrays = [np.array(w, dtype=np.int64) for _, w, _, _ in self.ops]
+        # the tape as one array of PlkOp records; a call adds its parameters
+        # (built op by op through ctypes a tape took 5 us per op, a tenth of a
+        # 26-qubit gradient and most of a small one)
+        n = len(self.ops)
+        counts = np.array([len(w) for _, w, _, _ in self.ops], dtype=np.int64)
+        starts = np.concatenate([[0], np.cumsum(counts)[:-1]]) if n else counts
+        self._wires = np.array([x for _, w, _, _ in self.ops for x in w] or [0], dtype=np.int64)
+        self._param_of = np.array([pi for _, _, _, pi in self.ops], dtype=np.int64)
+        self._records = np.zeros(max(1, n), dtype=np.dtype(
+            [("gate", "<i4"), ("nw", "<i4"), ("adj", "<i4"), ("np", "<i4"), ("w", "<u8"), ("p", "<u8"), ("m", "<u8")]))
+        if n:
+            self._records["gate"] = [g for g, _, _, _ in self.ops]
+            self._records["nw"] = counts
+            self._records["adj"] = [int(inv) for _, _, inv, _ in self.ops]
+            self._records["np"] = self._param_of >= 0
+            self._records["w"] = self._wires.ctypes.data + 8 * starts.astype(np.uint64)
+        self._trainable = np.flatnonzero(self._param_of >= 0)
 
     # -- helpers -----------------------------------------------------------
     def _tape(self, params: np.ndarray):
-        arr = (N.PlkOp * max(1, len(self.ops)))()
-        keep = []
-        for i, (g, _, inv, pi) in enumerate(self.ops):
-            w = self._wire_arrays[i]
-            p = np.array([params[pi] if pi >= 0 else 0.0], dtype=np.float64)
-            keep.append(p)
-            arr[i] = N.PlkOp(g, len(w), int(inv), 1 if pi >= 0 else 0, _ptr(w, C.c_int64), _ptr(p, C.c_double), None)
-        return arr, keep
+        """(PlkOp pointer, what it points to)"""
+        values = np.zeros(len(self._records))
+        if len(self._trainable):
+            values[self._trainable] = params[self._param_of[self._trainable]]
+        records = self._records.copy()
+        records["p"] = values.ctypes.data + 8 * np.arange(len(records), dtype=np.uint64)
+        return C.cast(records.ctypes.data, C.POINTER(N.PlkOp)), (records, values)
 
     def _stream(self):
         return torch.cuda.current_stream(self.device).cuda_stream
@@ -166,9 +181,8 @@ class AdjointCircuit:
             N.check(N.lib.plk_apply_pauli_sum(hl.h, lam.h, len(c), _ptr(c, C.c_double), _ptr(o, C.c_int64),
                                               _ptr(w, C.c_int64), l))
             arr, keep = self._tape(params)
-            tp_ops = [i for i, op in enumerate(self.ops) if op[3] >= 0]
-            tp = np.arange(len(tp_ops), dtype=np.int64)
-            jac = np.zeros(len(tp_ops))
+            tp = np.arange(len(self._trainable), dtype=np.int64)
+            jac = np.zeros(len(tp))
             harr = (C.c_void_p * 1)(hl.h.value)
             fn = N.lib.plk_adjoint_jacobian_inplace if inplace else N.lib.plk_adjoint_jacobian
             N.check(fn(lam.h, harr, 1, arr, len(self.ops), _ptr(tp, C.c_int64), len(tp), _ptr(jac, C.c_double)))
@@ -177,8 +191,7 @@ class AdjointCircuit:
             if inplace:
                 lam.free()
         grad = np.zeros(self.num_params)
-        for t, i in enumerate(tp_ops):
-            grad[self.ops[i][3]] += jac[t]
+        np.add.at(grad, self._param_of[self._trainable], jac)
         return grad
 
     def __call__(self, params: torch.Tensor) -> torch.Tensor:
