@@ -235,6 +235,15 @@ PLK_API int plk_adjoint_jacobian_inplace(plk_state lambda, plk_state *hlambda, i
                                          const plk_op *ops, int32_t num_ops, const int64_t *trainable,
                                          int32_t num_trainable, double *jac);
 
+/* The same Jacobian for observables that are one Pauli word each (observable o:
+ * coeffs[o] times the letters offsets[o] .. offsets[o+1]) without the caller
+ * forming H lambda: the sweep reads it off lambda, which is not modified.
+ * PLK_ERR_UNSUPPORTED when the tape or the free memory does not allow it (then
+ * form the states and call plk_adjoint_jacobian). */
+PLK_API int plk_adjoint_jacobian_pauli(plk_state lambda, int32_t num_obs, const double *coeffs, const int64_t *offsets,
+                                       const int64_t *wires, const char *paulis, const plk_op *ops, int32_t num_ops,
+                                       const int64_t *trainable, int32_t num_trainable, double *jac);
+
 /* ---- allocation-free expectation values ------------------------------ */
 /* No counterpart in the reference.  For callers that may not allocate device
  * memory — their device memory belongs to another allocator or to a fixed

@@ -185,13 +185,7 @@ static int adjoint_impl(plk_state lam, plk_state *hl, int nobs, const plk_op *op
     return PLK_OK;
 }
 
-} // namespace plk
-
-using namespace plk;
-
-extern "C" {
-
-static int adjoint_checks(plk_state lambda, plk_state *hlambda, int32_t nobs, const plk_op *ops, int32_t nops,
+int adjoint_checks(plk_state lambda, plk_state *hlambda, int32_t nobs, const plk_op *ops, int32_t nops,
                           const int64_t *trainable, int32_t ntp, double *jac) {
     PLK_TRY(check_state(lambda));
     if (ntp <= 0) PLK_FAIL(PLK_ERR_INVALID_ARG, "No trainable parameters provided.");
@@ -214,6 +208,12 @@ static int adjoint_checks(plk_state lambda, plk_state *hlambda, int32_t nobs, co
     }
     return PLK_OK;
 }
+
+} // namespace plk
+
+using namespace plk;
+
+extern "C" {
 
 // Runs the sweep with `work` as lambda (overwritten) and the observable states
 // moved onto its stream for the duration of the call.

@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kBThreads, BWD ? kBCtasBwd : kBCtasFwd)
         for (int i = lane; i < j.nacc; i += 32) row[i] = make_float2(0.0f, 0.0f);
     __syncthreads();
     const Pass ps(prog);
-    const Buffers bf{states + j.lam, states + j.lam, states + j.hl, 0, 0, !BWD && j.first_pass};
+    const Buffers bf{states + j.lam, states + j.lam, states + j.hl, 0, 0, !BWD && j.first_pass, false, 0, 0, 0};
     for (int t = 0; t < c.ntiles; t++) run_tile<AmpC64, kBR, BWD>(ps, bf, c.tile0 + t, j.T, L, M, row);
     if (BWD) {
         for (int i = tid; i < j.nacc; i += blockDim.x) {

@@ -109,6 +109,8 @@ template <class T> class AdjointJacobianGB {
             tape.push_back({g, (int32_t)w[i].size(), (int32_t)ops.getOpsInverses()[i], (int32_t)p[i].size(),
                             w[i].data(), p[i].data(), mat});
         }
+        std::vector<int64_t> tp(trainable.begin(), trainable.end());
+        if (!apply_operations && singleWords(ref_data, jac, obs, tape, tp)) return;
         StateVectorGB<T> lambda(ref_data);
         if (apply_operations) check(plk_apply_ops(lambda.handle(), tape.data(), (int32_t)tape.size()));
         // H_lambda states
@@ -124,10 +126,33 @@ template <class T> class AdjointJacobianGB {
             }
             hh.push_back(hl.back()->handle());
         }
-        std::vector<int64_t> tp(trainable.begin(), trainable.end());
         jac.assign(obs.size() * trainable.size(), 0.0);
         check(plk_adjoint_jacobian(lambda.handle(), hh.data(), (int32_t)hh.size(), tape.data(), (int32_t)tape.size(),
                                    tp.data(), (int32_t)tp.size(), jac.data()));
+    }
+
+  private:
+    // Observables of one Pauli word each need no states of their own.  False:
+    // some are not, or the library asks for the states.
+    static bool singleWords(const StateVectorGB<T> &lambda, std::vector<double> &jac,
+                            const std::vector<std::shared_ptr<ObservableGB<T>>> &obs, const std::vector<plk_op> &tape,
+                            const std::vector<int64_t> &tp) {
+        std::vector<double> c;
+        std::vector<int64_t> off{0}, w;
+        std::string letters;
+        for (const auto &ob : obs) {
+            const auto words = ob->pauliWords();
+            if (!words || words->size() != 1) return false;
+            c.push_back((*words)[0].coeff);
+            for (const size_t x : (*words)[0].wires) w.push_back((int64_t)x);
+            letters += (*words)[0].letters;
+            off.push_back((int64_t)w.size());
+        }
+        jac.assign(obs.size() * tp.size(), 0.0);
+        // any failure is met, and reported, by the general way
+        return plk_adjoint_jacobian_pauli(lambda.handle(), (int32_t)c.size(), c.data(), off.data(), w.data(),
+                                          letters.c_str(), tape.data(), (int32_t)tape.size(), tp.data(),
+                                          (int32_t)tp.size(), jac.data()) == PLK_OK;
     }
 };
 

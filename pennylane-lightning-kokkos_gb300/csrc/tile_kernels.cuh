@@ -50,6 +50,10 @@ struct Args {
     int nacc_all;      // accumulators of the whole program
     int in_df, out_df; // complex128: buffers hold double-float pairs on entry / exit
     double *part;      // [sweep][accumulator][gridDim.x]
+    // when set, H lambda of sweep y starts as the Pauli word i^ny (-1)^popcount(k & z) |k ^ x> on lam_src[y]
+    int words;
+    uint32_t wx[kMaxSweeps], wz[kMaxSweeps];
+    uint8_t wq[kMaxSweeps]; // number of Y letters
 };
 
 __device__ __forceinline__ f2x f2x_dup(float a) { return f2x_pack(a, a); }
@@ -555,10 +559,17 @@ struct Buffers {
     void *lam, *hl;
     int in_df, out_df; // complex128: double-float pairs on entry / exit
     bool from_zero;    // the state is |0...0> on entry, lam_src is not read
+    bool word;         // H lambda is a Pauli word on lam_src, hl is not read
+    uint32_t wx, wz, wq;
 };
 
 // All rounds of one tile; every thread of the CTA takes part.  L, M: the tile's
 // slots of lambda and H lambda; row: this warp's accumulators.
+__device__ __forceinline__ f2x times_i(f2x v) { return f2x_pack(-f2x_hi(v), f2x_lo(v)); }
+__device__ __forceinline__ AmpC128::V times_i(const AmpC128::V &v) { return {times_i(v.h), times_i(v.l)}; }
+__device__ __forceinline__ f2x negate(f2x v) { return v ^ 0x8000000080000000ull; }
+__device__ __forceinline__ AmpC128::V negate(const AmpC128::V &v) { return {negate(v.h), negate(v.l)}; }
+
 template <class A, int R, bool BWD>
 __device__ __forceinline__ void run_tile(const Pass &ps, const Buffers &bf, int tile, int T, unsigned char *L,
                                          unsigned char *M, float2 *row) {
@@ -599,7 +610,16 @@ __device__ __forceinline__ void run_tile(const Pass &ps, const Buffers &bf, int 
                 const uint32_t i = g ^ ((j & 3) == 3 ? g01 : (j & 1) ? g0 : (j & 2) ? g1 : 0u) ^
                                    ((j & 12) == 12 ? g23 : (j & 4) ? g2 : (j & 8) ? g3 : 0u);
                 v[j] = bf.from_zero ? basis_amp(i, V{}) : load_amp(lam, i, bf.in_df, V{});
-                if (BWD) h[j] = load_amp(hl, i, bf.in_df, V{});
+                if (BWD) {
+                    if (bf.word) {
+                        const uint32_t k = i ^ bf.wx;
+                        h[j] = load_amp(lam, k, bf.in_df, V{});
+                        if (bf.wq & 1u) h[j] = times_i(h[j]);
+                        if ((bf.wq >> 1 ^ __popc(k & bf.wz)) & 1u) h[j] = negate(h[j]);
+                    } else {
+                        h[j] = load_amp(hl, i, bf.in_df, V{});
+                    }
+                }
             }
         } else {
 #pragma unroll
@@ -712,7 +732,8 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_tile(const __grid_constant__ 
         for (int i = lane; i < a.nacc; i += 32) row[i] = make_float2(0.0f, 0.0f);
     __syncthreads();
     const Pass ps(prog);
-    const Buffers bf{a.lam_src[blockIdx.y], a.lam[blockIdx.y], a.hl[blockIdx.y], a.in_df, a.out_df, false};
+    const Buffers bf{a.lam_src[blockIdx.y], a.lam[blockIdx.y], a.hl[blockIdx.y], a.in_df, a.out_df, false,
+                     BWD && a.words, a.wx[blockIdx.y], a.wz[blockIdx.y], a.wq[blockIdx.y]};
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) run_tile<A, R, BWD>(ps, bf, tile, a.T, L, M, row);
     if (BWD) {
         for (int i = tid; i < a.nacc; i += blockDim.x) {

@@ -56,6 +56,12 @@ static int tile_bits(int nq, int dtype, bool bwd) {
     return std::min(T, nq);
 }
 
+struct Word { // coeff i^ny (-1)^popcount(k & z) |k ^ x>
+    uint32_t x, z;
+    int ny;
+    double coeff;
+};
+
 static Options options(int nq, int dtype, bool bwd) {
     Options o;
     o.T = tile_bits(nq, dtype, bwd);
@@ -76,8 +82,11 @@ static int check_program(const TileProgram &P, int amp_bytes) {
 
 // Runs P on nsweep (lambda, H lambda) pairs on stream st.  Backward, the
 // Jacobian rows go to jac_host (row-major [nsweep][nslots]; synchronizes).
+// words: H lambda of each sweep starts as that Pauli word on lam_src instead of
+// what hl holds.
 static int run(const TileProgram &P, int dtype, int device, cudaStream_t st, const void *const *lam_src,
-               void *const *lam, void *const *hl, int nsweep, int nslots, double *jac_host) {
+               void *const *lam, void *const *hl, int nsweep, int nslots, double *jac_host,
+               const Word *words = nullptr) {
     DeviceCtx *d = nullptr;
     PLK_TRY(device_ctx(device, &d));
     const bool c64 = dtype == PLK_C64;
@@ -127,6 +136,11 @@ static int run(const TileProgram &P, int dtype, int device, cudaStream_t st, con
         a.lam_src[y] = lam_src[y];
         a.lam[y] = lam[y];
         a.hl[y] = P.bwd ? hl[y] : nullptr;
+        if (words) {
+            a.wx[y] = words[y].x;
+            a.wz[y] = words[y].z;
+            a.wq[y] = (uint8_t)(words[y].ny & 3);
+        }
     }
     a.T = P.T;
     a.ntiles = ntiles;
@@ -139,6 +153,7 @@ static int run(const TileProgram &P, int dtype, int device, cudaStream_t st, con
         a.prog_bytes = h.bytes;
         a.nacc = h.nacc;
         a.in_df = i > 0;
+        a.words = words && i == 0;
         a.out_df = i + 1 < P.passes.size();
         const size_t smem = smem_bytes(c64 ? 8 : 16, P.bwd, P.T, h.bytes, h.nacc, threads);
         if (c64) PLK_TRY(launch_c64(P.bwd, a, grid, threads, smem, st));
@@ -197,12 +212,11 @@ int apply_ops(plk_state s, const plk_op *ops, int nops, bool &handled) {
     return run(P, s->dtype, s->device, s->stream, src, dst, nullptr, 1, 0, nullptr);
 }
 
-// Backward sweeps of all observables; lam is the working copy of the forward
-// state (overwritten by the last group of sweeps).
-int adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops, const int64_t *tp, int ntp,
-            double *jac, bool &handled) {
-    handled = false;
-    if (!usable(lam) || ntp <= 0 || nobs < 1) return PLK_OK;
+// The backward program of a tape; ok stays false when an op is not of this path.
+static int compile_backward(plk_state lam, const plk_op *ops, int nops, const int64_t *tp, int ntp, TileProgram &P,
+                            int &swept, bool &ok) {
+    ok = false;
+    swept = 0;
     int num_param_ops = 0;
     for (int i = 0; i < nops; i++)
         if (ops[i].num_params > 0) num_param_ops++;
@@ -211,7 +225,7 @@ int adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops
     Compiler c(lam->nq, true, options(lam->nq, lam->dtype, true));
     Lowered L;
     long current_param_idx = num_param_ops - 1;
-    int tp_it = ntp - 1, swept = 0;
+    int tp_it = ntp - 1;
     for (int i = nops - 1; i >= 0 && tp_it >= 0; i--) {
         const plk_op &op = ops[i];
         if (op.num_params > 1) return PLK_OK; // rejected by the reference; the per-op path reports it
@@ -230,11 +244,27 @@ int adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops
         if (trainable) tp_it--;
         if (op.num_params > 0) current_param_idx--;
     }
+    ok = c.compile(P) && !P.passes.empty();
+    return PLK_OK;
+}
+
+// 4 state moves per pass and observable, against 2 (1 + nobs) per op for the
+// op-at-a-time kernel that carries every H lambda along
+static bool worth_it(const TileProgram &P, int nobs, int swept) {
+    return nobs == 1 || 4.0 * nobs * P.passes.size() <= 2.0 * (1.0 + nobs) * swept;
+}
+
+// Backward sweeps of all observables; lam is the working copy of the forward
+// state (overwritten).
+int adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops, const int64_t *tp, int ntp,
+            double *jac, bool &handled) {
+    handled = false;
+    if (!usable(lam) || ntp <= 0 || nobs < 1) return PLK_OK;
     TileProgram P;
-    if (!c.compile(P) || P.passes.empty()) return PLK_OK;
-    // 4 state moves per pass and observable, against 2 (1 + nobs) per op for
-    // the op-at-a-time kernel that carries every H lambda along
-    if (nobs > 1 && 4.0 * nobs * P.passes.size() > 2.0 * (1.0 + nobs) * swept) return PLK_OK;
+    int swept = 0;
+    bool ok = false;
+    PLK_TRY(compile_backward(lam, ops, nops, tp, ntp, P, swept, ok));
+    if (!ok || !worth_it(P, nobs, swept)) return PLK_OK;
     // several sweeps start from lambda: each works on its own copy
     const size_t bytes = lam->length * amp_bytes(lam->dtype);
     int group = std::min(nobs, kMaxSweeps);
@@ -266,5 +296,85 @@ int adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops
     return PLK_OK;
 }
 
+// Observables that are one Pauli word each: H lambda is never stored, the first
+// pass reads it as the permuted, signed lambda (which is not modified).
+static int adjoint_words(plk_state lam, const std::vector<Word> &words, const plk_op *ops, int nops, const int64_t *tp,
+                         int ntp, double *jac, bool &handled) {
+    handled = false;
+    const int nobs = (int)words.size();
+    if (!usable(lam) || ntp <= 0 || nobs < 1) return PLK_OK;
+    TileProgram P;
+    int swept = 0;
+    bool ok = false;
+    PLK_TRY(compile_backward(lam, ops, nops, tp, ntp, P, swept, ok));
+    if (!ok || !worth_it(P, nobs, swept)) return PLK_OK;
+    DeviceCtx *d = nullptr;
+    PLK_TRY(device_ctx(lam->device, &d));
+    const size_t bytes = std::max<size_t>(256, lam->length * amp_bytes(lam->dtype));
+    const int group =
+        (int)std::min<size_t>(std::min(nobs, kMaxSweeps), std::max<size_t>(1, ((size_t)4 << 30) / (2 * bytes)));
+    PoolBuf buf(lam->stream);
+    if (cudaMallocFromPoolAsync(&buf.p, 2 * bytes * group, d->pool, lam->stream) != cudaSuccess) {
+        cudaGetLastError();
+        buf.p = nullptr;
+        return PLK_OK; // the caller has ways that need less
+    }
+    handled = true;
+    for (int o0 = 0; o0 < nobs; o0 += group) {
+        const int n = std::min(group, nobs - o0);
+        const void *src[kMaxSweeps];
+        void *dst[kMaxSweeps], *h[kMaxSweeps];
+        for (int y = 0; y < n; y++) {
+            src[y] = lam->data;
+            dst[y] = buf.as<char>() + 2 * bytes * y;
+            h[y] = buf.as<char>() + 2 * bytes * y + bytes;
+        }
+        PLK_TRY(run(P, lam->dtype, lam->device, lam->stream, src, dst, h, n, ntp, jac + (size_t)o0 * ntp, &words[o0]));
+    }
+    for (int o = 0; o < nobs; o++) // the sweeps ran on the bare words
+        for (int t = 0; t < ntp; t++) jac[(size_t)o * ntp + t] *= words[o].coeff;
+    return PLK_OK;
+}
+
 } // namespace tile
+
+int adjoint_checks(plk_state lambda, plk_state *hlambda, int32_t nobs, const plk_op *ops, int32_t nops,
+                   const int64_t *trainable, int32_t ntp, double *jac);
+
 } // namespace plk
+
+using namespace plk;
+
+extern "C" {
+
+PLK_API int plk_adjoint_jacobian_pauli(plk_state lambda, int32_t num_obs, const double *coeffs, const int64_t *offsets,
+                                       const int64_t *wires, const char *paulis, const plk_op *ops, int32_t num_ops,
+                                       const int64_t *trainable, int32_t num_trainable, double *jac) {
+    PLK_TRY(adjoint_checks(lambda, nullptr, 0, ops, num_ops, trainable, num_trainable, jac));
+    if (num_obs < 1 || !coeffs || !offsets) PLK_FAIL(PLK_ERR_INVALID_ARG, "bad Pauli-word arguments");
+    PLK_CUDA(cudaSetDevice(lambda->device));
+    std::vector<tile::Word> words;
+    for (int o = 0; o < num_obs; o++) {
+        tile::Word w{0, 0, 0, coeffs[o]};
+        for (int64_t j = offsets[o]; j < offsets[o + 1]; j++) {
+            if (!wires || !paulis || wires[j] < 0 || wires[j] >= lambda->nq || lambda->nq > 32)
+                PLK_FAIL(PLK_ERR_INVALID_ARG, "Pauli word wire out of range");
+            const uint32_t bit = 1u << (lambda->nq - 1 - wires[j]);
+            if ((w.x | w.z) & bit) PLK_FAIL(PLK_ERR_INVALID_ARG, "repeated wire in a Pauli word");
+            switch (paulis[j]) {
+            case 'I': break;
+            case 'X': w.x |= bit; break;
+            case 'Y': w.x |= bit; w.z |= bit; w.ny++; break;
+            case 'Z': w.z |= bit; break;
+            default: PLK_FAIL(PLK_ERR_INVALID_ARG, std::string("bad Pauli letter ") + paulis[j]);
+            }
+        }
+        words.push_back(w);
+    }
+    bool handled = false;
+    PLK_TRY(tile::adjoint_words(lambda, words, ops, num_ops, trainable, num_trainable, jac, handled));
+    if (!handled) PLK_FAIL(PLK_ERR_UNSUPPORTED, "this tape's sweep does not start from Pauli words");
+    return PLK_OK;
+}
+
+} // extern "C"

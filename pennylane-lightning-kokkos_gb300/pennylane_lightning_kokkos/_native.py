@@ -101,6 +101,8 @@ _SIGS = {
                              C.c_int),
     "plk_adjoint_jacobian_inplace": ([_vp, C.POINTER(_vp), C.c_int32, C.POINTER(PlkOp), C.c_int32, _i64p, C.c_int32,
                                       _dp], C.c_int),
+    "plk_adjoint_jacobian_pauli": ([_vp, C.c_int32, _dp, _i64p, _i64p, C.c_char_p, C.POINTER(PlkOp), C.c_int32, _i64p,
+                                    C.c_int32, _dp], C.c_int),
     "plk_expval_pauliz_noalloc": ([_vp, C.c_int32, C.c_int32, C.c_int32, _i64p, _dp, _vp], C.c_int),
     "plk_set_window_path": ([C.c_int32], C.c_int),
     "plk_get_window_path": ([_i32p], C.c_int),

@@ -65,3 +65,42 @@ def test_index_maps_only(dtype):
     else: # 48 of a double's 53 bits pass through the sweep
         np.testing.assert_allclose(got, ref, rtol=2.0 ** -46, atol=0)
     del keep
+
+
+@pytest.mark.parametrize("dtype", [N.PLK_C64, N.PLK_C128])
+@pytest.mark.parametrize("nq", [4, 8, 11, 12, 14])
+def test_jacobian_of_pauli_words(nq, dtype):
+    """Sweeps that read H lambda off lambda: words with every letter, none, and
+    more than one launch holds (32)."""
+    import ctypes as C
+
+    from abi import f64, i64
+
+    rng = np.random.default_rng(900 + nq)
+    ops = random_ops(nq, 60, rng, single_param=True)
+    npar = sum(1 for o in ops if o[3])
+    trainable = sorted(int(x) for x in rng.choice(npar, npar // 2 + 1, replace=False))
+    words = [(1.0, [w], "Z") for w in range(nq)] + [(0.7, [], "")]
+    while len(words) < (35 if nq == 8 else nq + 6):
+        k = int(rng.integers(1, nq + 1))
+        words.append((float(rng.standard_normal()), [int(w) for w in rng.choice(nq, k, replace=False)],
+                      "".join(str(x) for x in rng.choice(list("XYZI"), k))))
+    name = {"X": "PauliX", "Y": "PauliY", "Z": "PauliZ", "I": "Identity"}
+    obs = [("hamiltonian", [c], [("tensor", [("named", name[l], [w]) for w, l in zip(ws, ls)] or
+                                  [("named", "Identity", [0])])]) for c, ws, ls in words]
+    psi = rand_state(nq, rng)
+    ref = O.adjoint_jacobian(psi, obs, ops, trainable)
+    s = State.from_array(psi, dtype)
+    before = s.get()
+    arr, keep = make_ops(ops)
+    c, cp = f64([w[0] for w in words])
+    off, offp = i64(np.cumsum([0] + [len(w[1]) for w in words]))
+    wi, wp = i64([x for w in words for x in w[1]])
+    tp, tpp = i64(trainable)
+    jac = np.zeros((len(words), len(trainable)))
+    N.check(N.lib.plk_adjoint_jacobian_pauli(s.h, len(words), cp, offp, wp, "".join(w[2] for w in words).encode(), arr,
+                                             len(ops), tpp, len(tp), jac.ctypes.data_as(C.POINTER(C.c_double))))
+    np.testing.assert_allclose(jac, ref, atol=JTOL[dtype], rtol=0)
+    np.testing.assert_array_equal(s.get(), before)
+    s.close()
+    del keep
