@@ -492,19 +492,19 @@ __device__ __forceinline__ void step_cry(typename A::V (&v)[1 << R], typename A:
 // truncating split of df.cuh leaves a low part of up to 2^-23 of the high part,
 // always of its sign, and what it cuts off and the low parts' dropped products
 // add up to a bias of about 2^-48 of a sum's magnitudes (seen in energies whose
-// words nearly cancel: 8e-13 against 8e-14).
+// words nearly cancel: 8e-13 against 8e-14).  A float's exponent is the double's
+// less 896, which is its low eight bits with the top one flipped; the 29 bits that
+// the high part leaves out are converted as an integer and scaled by the high
+// part's power of two.  (Assembled from shifted fields on the integer pipe the
+// split took twice the instructions, a third of a pass over a Pauli sum.)
 __device__ __forceinline__ DF df_split_near(double x) {
     const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    const unsigned hw = (unsigned)(u >> 32), lw = (unsigned)u, sign = hw & 0x80000000u;
-    const int ef = (int)((hw >> 20) & 0x7ffu) - 896, el = ef - 23; // float exponents of hi and of its last place
-    const unsigned top = ((hw & 0xfffffu) << 3) | (lw >> 29);
-    const unsigned next = ((lw & 0x1fffffffu) + 32u) >> 6; // up to 2^23
-    const float hi = (ef >= 1 && ef <= 254) ? __uint_as_float(sign | ((unsigned)ef << 23) | top) : 0.0f;
-    float lo = 0.0f;
-    if (el >= 1 && el <= 253) { // (1 + next / 2^23) 2^E - 2^E, exact
-        const float f = __uint_as_float(((unsigned)el << 23) + next), g = __uint_as_float((unsigned)el << 23);
-        lo = __uint_as_float(__float_as_uint(__fsub_rn(f, g)) | sign);
-    }
+    const unsigned hw = (unsigned)(u >> 32), lw = (unsigned)u;
+    const unsigned mag = (__funnelshift_l(lw, hw, 3) ^ 0x40000000u) & 0x7fffffffu;
+    const bool fits = 2u * hw - (897u << 21) < (254u << 21); // a normal float; else 0
+    const float hi = fits ? __uint_as_float(mag | (hw & 0x80000000u)) : 0.0f;
+    const float power = __uint_as_float(__float_as_uint(hi) & 0xff800000u);
+    const float lo = __fmul_rn(__fmul_rn(__uint2float_rn(lw & 0x1fffffffu), 0x1p-52f), power);
     const float s = __fadd_rn(hi, lo);
     return {s, __fsub_rn(lo, __fsub_rn(s, hi))};
 }
