@@ -59,10 +59,11 @@ constexpr int kPT = 12, kPR = 4, kPA = 1 << kPR; // tile bits, register bits
 constexpr int kPer = 1 << (kPT - kPR);           // slots between register indices, whatever T is
 
 // From how many words with the same x and factor on the coefficients are formed
-// per amplitude (instructions per amplitude, from the code: a transform 21 per 16
-// amplitudes or 11 per eight pairs; a word 16 in complex128, 6 in complex64, in an
-// expectation value 10 and 4).
-constexpr int kManyApplyC64 = 7, kManyApplyC128 = 3, kManyExpvalC64 = 6, kManyExpvalC128 = 3;
+// per amplitude.  24 qubits, ten patterns of n words, us through a transform / word
+// by word: application complex64 n = 6 465 / 406, 8 508 / 501, 10 540 / 593,
+// complex128 3 743 / 663, 4 756 / 821; expectation value complex64 5 389 / 357,
+// 6 384 / 407, complex128 2 423 / 350, 3 437 / 463.
+constexpr int kManyApplyC64 = 9, kManyApplyC128 = 4, kManyExpvalC64 = 6, kManyExpvalC128 = 3;
 
 struct alignas(16) Item {
     uint32_t w;   // bits 0-15 x as a byte offset in the tile (exclusive or), 16-19 sign bits on register

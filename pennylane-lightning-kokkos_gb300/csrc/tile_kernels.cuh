@@ -455,9 +455,9 @@ __device__ __forceinline__ void step_index(typename A::V (&v)[1 << R], typename 
 // Rotation of register bit B: sums first (both states as they are before it)
 template <class A, int R, bool BWD, int B>
 __device__ __forceinline__ void step_ry(typename A::V (&v)[1 << R], typename A::V (&h)[1 << R], const TileStage &st,
-                                        DF (&y)[4], DF (&x)[4]) {
+                                        uint32_t ry, DF (&y)[4], DF (&x)[4]) {
     if constexpr (B < R) {
-        if (!(st.ry >> B & 1)) return;
+        if (!(ry >> B & 1)) return;
         if (BWD) {
             if (st.acc_y[B] >= 0) y[B] = sum_y<1 << R, B, false>(v, h, 0u);
             if (st.acc_x[B] >= 0) x[B] = sum_x<1 << R, B>(v, h);
@@ -553,6 +553,37 @@ struct Pass {
           index(reinterpret_cast<const TileIndex *>(p + hd.off_index)), tab(p + hd.off_tab) {}
 };
 
+// The fields of a stage and a round that every thread needs, in one shared-memory
+// read each: read one by one, each branch waited for its own.
+struct StageHead {
+    uint32_t ry, table, special, sums, tab, zsel;
+    int acc_z;
+    __device__ __forceinline__ explicit StageHead(const TileStage &st) {
+        const uint4 w = *reinterpret_cast<const uint4 *>(&st.ry);
+        ry = w.x & 255u;
+        table = w.x >> 8 & 255u;
+        special = w.x >> 16 & 255u;
+        sums = w.x >> 24;
+        tab = w.y & 0xffffu;
+        zsel = w.y >> 16;
+        acc_z = (int16_t)(w.z & 0xffffu);
+    }
+};
+struct RoundHead {
+    uint32_t r0, r1, r2, r3, xorc, stage0, nstages, ev0;
+    __device__ __forceinline__ explicit RoundHead(const TileRound &q) {
+        const uint4 w = *reinterpret_cast<const uint4 *>(q.rcol);
+        r0 = w.x & 0xffffu;
+        r1 = w.x >> 16;
+        r2 = w.y & 0xffffu;
+        r3 = w.y >> 16;
+        xorc = w.z & 0xffffu;
+        stage0 = w.z >> 16;
+        nstages = w.w & 0xffffu;
+        ev0 = w.w >> 16;
+    }
+};
+
 // state buffers of a sweep
 struct Buffers {
     const void *lam_src;
@@ -586,14 +617,15 @@ __device__ __forceinline__ void run_tile(const Pass &ps, const Buffers &bf, int 
     uint32_t ev = 0;
     for (int r = 0; r < nrounds; r++) {
         const TileRound &q = ps.rounds[r];
+        const RoundHead rh(q);
         uint32_t gev = base;
         for (int k = 0; k < q.nev; k++)
-            if (base >> ps.events[q.ev0 + k].bit & 1u) {
-                ev ^= ps.events[q.ev0 + k].mask;
-                gev ^= ps.events[q.ev0 + k].gmask;
+            if (base >> ps.events[rh.ev0 + k].bit & 1u) {
+                ev ^= ps.events[rh.ev0 + k].mask;
+                gev ^= ps.events[rh.ev0 + k].gmask;
             }
-        const uint32_t o = q.lo[lane] ^ q.hi[warp] ^ q.xorc ^ ev;
-        const uint32_t r0 = q.rcol[0], r1 = q.rcol[1], r2 = q.rcol[2], r3 = q.rcol[3];
+        const uint32_t o = q.lo[lane] ^ q.hi[warp] ^ rh.xorc ^ ev;
+        const uint32_t r0 = rh.r0, r1 = rh.r1, r2 = rh.r2, r3 = rh.r3;
         const uint32_t r01 = r0 ^ r1, r23 = r2 ^ r3; // one three-input operation per slot
         auto slot = [&](int j) {
             return o ^ ((j & 3) == 3 ? r01 : (j & 1) ? r0 : (j & 2) ? r1 : 0u) ^
@@ -630,50 +662,66 @@ __device__ __forceinline__ void run_tile(const Pass &ps, const Buffers &bf, int 
         }
         uint32_t gi = base;
         if (q.idx != 0xffffu) gi |= ps.index[q.idx].lo[lane] | ps.index[q.idx].hi[warp];
-        for (int k = 0; k < q.nstages; k++) {
-            const TileStage &st = ps.stages[q.stage0 + k];
+        for (int k = 0; k < (int)rh.nstages; k++) {
+            const TileStage &st = ps.stages[rh.stage0 + k];
+            const StageHead f(st);
             DF y[8] = {}; // Y sums by bit, then Z sums by bit
             DF x[4] = {};
             bool zbits = false;
-            if (BWD && (st.table & 1)) {
-                zbits = (st.zsel & ~0x0116u) == 0;
+            if (BWD && (f.table & 1)) {
+                zbits = (f.zsel & ~0x0116u) == 0;
                 if (zbits) walsh_bits<A, R>(v, h, y + 4);
-                else walsh_all<A, R>(v, h, st.zsel, st.acc_z, row, lane);
+                else walsh_all<A, R>(v, h, f.zsel, f.acc_z, row, lane);
             }
-            if (st.table & 2) {
-                const auto *e = reinterpret_cast<const typename Form<A>::E *>(ps.tab) + st.tab;
+            if (f.table & 2) {
+                if constexpr (A::kBytes == 8) { // two entries a read
+                    const float4 *e = reinterpret_cast<const float4 *>(ps.tab + f.tab * sizeof(float2));
 #pragma unroll
-                for (int j = 0; j < NA; j++) {
-                    const auto z = e[j];
-                    phase(v[j], z);
-                    if (BWD) phase(h[j], z);
+                    for (int j = 0; j < NA; j += 2) {
+                        const float4 z = e[j / 2];
+                        const float2 z0 = make_float2(z.x, z.y), z1 = make_float2(z.z, z.w);
+                        phase(v[j], z0);
+                        phase(v[j + 1], z1);
+                        if (BWD) {
+                            phase(h[j], z0);
+                            phase(h[j + 1], z1);
+                        }
+                    }
+                } else {
+                    const auto *e = reinterpret_cast<const typename Form<A>::E *>(ps.tab) + f.tab;
+#pragma unroll
+                    for (int j = 0; j < NA; j++) {
+                        const auto z = e[j];
+                        phase(v[j], z);
+                        if (BWD) phase(h[j], z);
+                    }
                 }
             }
             {
                 DF(&y4)[4] = reinterpret_cast<DF(&)[4]>(y);
-                step_ry<A, R, BWD, 0>(v, h, st, y4, x);
-                step_ry<A, R, BWD, 1>(v, h, st, y4, x);
-                step_ry<A, R, BWD, 2>(v, h, st, y4, x);
-                step_ry<A, R, BWD, 3>(v, h, st, y4, x);
+                step_ry<A, R, BWD, 0>(v, h, st, f.ry, y4, x);
+                step_ry<A, R, BWD, 1>(v, h, st, f.ry, y4, x);
+                step_ry<A, R, BWD, 2>(v, h, st, f.ry, y4, x);
+                step_ry<A, R, BWD, 3>(v, h, st, f.ry, y4, x);
             }
             if (BWD) {
-                if (zbits || (st.sums & 1)) {
-                    int id[8], next = st.acc_z;
+                if (zbits || (f.sums & 1)) {
+                    int id[8], next = f.acc_z;
 #pragma unroll
                     for (int b = 0; b < 4; b++) {
-                        id[b] = (st.ry >> b & 1) ? st.acc_y[b] : -1;
-                        id[4 + b] = (zbits && (st.zsel >> (1 << b) & 1)) ? next++ : -1;
+                        id[b] = (f.ry >> b & 1) ? st.acc_y[b] : -1;
+                        id[4 + b] = (zbits && (f.zsel >> (1 << b) & 1)) ? next++ : -1;
                     }
                     warp_sums<8>(y, id, row, lane);
                 }
-                if (st.sums & 2) {
+                if (f.sums & 2) {
                     int id[4];
 #pragma unroll
-                    for (int b = 0; b < 4; b++) id[b] = (st.ry >> b & 1) ? st.acc_x[b] : -1;
+                    for (int b = 0; b < 4; b++) id[b] = (f.ry >> b & 1) ? st.acc_x[b] : -1;
                     warp_sums<4>(x, id, row, lane);
                 }
             }
-            if (st.special == TS_CRY) {
+            if (f.special == TS_CRY) {
                 const uint32_t act = (gi & st.cmask) == st.cval ? st.jact : 0u;
                 DF c = {0.0f, 0.0f};
                 switch (st.bit) {
@@ -686,7 +734,7 @@ __device__ __forceinline__ void run_tile(const Pass &ps, const Buffers &bf, int 
                     c = warp_sum(c);
                     if (lane == 0) acc_add(row, st.sacc, c);
                 }
-            } else if (st.special != TS_NONE) {
+            } else if (f.special != TS_NONE) {
                 step_index<A, R, BWD>(v, h, st, ps.index[q.idx], gi, ps.tab, row, lane);
             }
         }

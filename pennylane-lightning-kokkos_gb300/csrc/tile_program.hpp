@@ -83,6 +83,7 @@ struct alignas(16) TileStage { // 144 bytes
     uint32_t pad2[4];
 };
 static_assert(sizeof(TileStage) == 144, "stage size");
+static_assert(offsetof(TileStage, ry) == 80 && offsetof(TileStage, stab) == 94, "ry .. stab are read as 16 bytes");
 
 struct alignas(16) TileRound { // 128 bytes
     uint16_t lo[32]; // byte offset in the tile of lane bits,
@@ -95,6 +96,7 @@ struct alignas(16) TileRound { // 128 bytes
     uint16_t pad[6];
 };
 static_assert(sizeof(TileRound) == 128, "round size");
+static_assert(offsetof(TileRound, rcol) == 96 && offsetof(TileRound, ev0) == 110, "rcol .. ev0 are read as 16 bytes");
 
 struct TileEvent { // when state bit `bit` of the tile's base is set, the map's constant is flipped
     uint16_t mask, bit; // byte offset
@@ -1491,7 +1493,7 @@ class Compiler {
                             for (double x : e.table) o.tab.push_back((float)x);
                             cur.sacc = acc(Terms{Term{e.slot, e.coef}});
                         }
-                        while (o.tab.size() % (o_.amp_bytes / sizeof(float))) o.tab.push_back(0.0f);
+                        while (o.tab.size() % 4) o.tab.push_back(0.0f); // tables are read 16 bytes at a time
                     }
                 }
             }
