@@ -332,26 +332,46 @@ __device__ __forceinline__ DF plus(DF a, DF b) {
     df_add(b.hi, b.lo, a.hi, a.lo);
     return a;
 }
-// Sums of N = 4 or 8 values over the warp, added to accumulators id[] (-1:
-// none).  Each of the first exchanges halves the number of values a lane
-// carries: eight sums take 9 exchanges instead of 40.
-template <int N> __device__ __forceinline__ void warp_sums(DF (&x)[N], const int (&id)[N], float2 *row, int lane) {
-    int k = 0; // which value this lane ends up with
+__device__ __forceinline__ f2x shfl(f2x a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+// Sums of N = 4 or 8 values over the warp.  Each of the first exchanges halves the
+// number of values a lane carries (eight sums take 9 exchanges instead of 40), two
+// values to an instruction while there are two.  The lane ends up with value k.
+template <int N> __device__ __forceinline__ DF warp_sums(const DF (&x)[N], int lane, int &k) {
+    f2x h[N / 2], l[N / 2];
+#pragma unroll
+    for (int i = 0; i < N / 2; i++) {
+        h[i] = f2x_pack(x[2 * i].hi, x[2 * i + 1].hi);
+        l[i] = f2x_pack(x[2 * i].lo, x[2 * i + 1].lo);
+    }
+    k = 0;
     int o = 16;
 #pragma unroll
-    for (int n = N / 2; n; n >>= 1, o >>= 1) {
+    for (int n = N / 4; n; n >>= 1, o >>= 1) {
         const bool up = lane & o;
 #pragma unroll
-        for (int i = 0; i < n; i++) x[i] = plus(pick(up, x[i + n], x[i]), shfl(pick(up, x[i], x[i + n]), o));
-        k += up ? n : 0;
+        for (int i = 0; i < n; i++) {
+            const f2x ah = up ? h[i] : h[i + n], al = up ? l[i] : l[i + n];
+            if (up) {
+                h[i] = h[i + n];
+                l[i] = l[i + n];
+            }
+            const f2x bh = shfl(ah, o), s = f2x_add(h[i], bh), bb = f2x_sub(s, h[i]);
+            const f2x t = f2x_add(f2x_sub(h[i], f2x_sub(s, bb)), f2x_sub(bh, bb));
+            l[i] = f2x_add(l[i], f2x_add(t, shfl(al, o)));
+            h[i] = s;
+        }
+        k += up ? 2 * n : 0;
     }
-    DF t = x[0];
+    const bool up = lane & o;
+    const DF a = {f2x_lo(h[0]), f2x_lo(l[0])}, b = {f2x_hi(h[0]), f2x_hi(l[0])};
+    DF t = plus(pick(up, b, a), shfl(pick(up, a, b), o));
+    k += up ? 1 : 0;
 #pragma unroll
     for (int q = 16 / N; q; q >>= 1) t = plus(t, shfl(t, q));
-    int mine = id[0];
-#pragma unroll
-    for (int i = 1; i < N; i++)
-        if (k == i) mine = id[i];
+    return t;
+}
+// the warp's sums added to accumulators, `mine` for the value this lane has (-1: none)
+template <int N> __device__ __forceinline__ void acc_sums(float2 *row, int lane, int mine, DF t) {
     if ((lane & (32 / N - 1)) == 0 && mine >= 0) acc_add(row, mine, t);
 }
 
@@ -401,13 +421,13 @@ __device__ __forceinline__ void walsh_all(const typename A::V (&v)[1 << R], cons
     for (int g = 0; g < NA / 4; g++)
         if (zsel >> (4 * g) & 15u) {
             DF x[4];
-            int id[4];
 #pragma unroll
-            for (int m = 0; m < 4; m++) {
-                x[m] = c[4 * g + m];
-                id[m] = (zsel >> (4 * g + m) & 1) ? next++ : -1;
-            }
-            warp_sums<4>(x, id, row, lane);
+            for (int m = 0; m < 4; m++) x[m] = c[4 * g + m];
+            const uint32_t z = zsel >> (4 * g) & 15u;
+            int k;
+            const DF t = warp_sums<4>(x, lane, k);
+            acc_sums<4>(row, lane, z >> k & 1 ? next + __popc(z & ((1u << k) - 1u)) : -1, t);
+            next += __popc(z);
         }
 }
 
@@ -706,19 +726,16 @@ __device__ __forceinline__ void run_tile(const Pass &ps, const Buffers &bf, int 
             }
             if (BWD) {
                 if (zbits || (f.sums & 1)) {
-                    int id[8], next = f.acc_z;
-#pragma unroll
-                    for (int b = 0; b < 4; b++) {
-                        id[b] = (f.ry >> b & 1) ? st.acc_y[b] : -1;
-                        id[4 + b] = (zbits && (f.zsel >> (1 << b) & 1)) ? next++ : -1;
-                    }
-                    warp_sums<8>(y, id, row, lane);
+                    int k;
+                    const DF t = warp_sums<8>(y, lane, k);
+                    // acc_y, then acc_zb
+                    const unsigned char *ids = reinterpret_cast<const unsigned char *>(&st) + offsetof(TileStage, acc_y);
+                    acc_sums<8>(row, lane, reinterpret_cast<const int16_t *>(ids)[k], t);
                 }
                 if (f.sums & 2) {
-                    int id[4];
-#pragma unroll
-                    for (int b = 0; b < 4; b++) id[b] = (f.ry >> b & 1) ? st.acc_x[b] : -1;
-                    warp_sums<4>(x, id, row, lane);
+                    int k;
+                    const DF t = warp_sums<4>(x, lane, k);
+                    acc_sums<4>(row, lane, st.acc_x[k], t);
                 }
             }
             if (f.special == TS_CRY) {

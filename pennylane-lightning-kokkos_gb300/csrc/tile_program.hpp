@@ -63,7 +63,7 @@ enum SpecialKind : uint8_t { TS_NONE = 0, TS_CRY = 1, TS_DIAG = 2, TS_PAR = 3 };
 // special step.
 struct alignas(16) TileStage { // 144 bytes
     float rot[4][4]; // bit b: complex64 the shears t, s as t.hi t.lo s.hi s.lo; complex128 t = s / c as t.hi t.lo
-    int16_t acc_y[4], acc_x[4]; // accumulators of Im <h|Y|v>, Im <h|X|v> (-1: none)
+    int16_t acc_y[4], acc_zb[4]; // accumulators of Im <h|Y|v> by bit, of the Walsh sums when all are of single bits (-1: none)
     uint8_t ry;      // bits that turn
     uint8_t table;   // bit 0: sums wanted (zsel), bit 1: phases to apply
     uint8_t special; // SpecialKind
@@ -80,10 +80,12 @@ struct alignas(16) TileStage { // 144 bytes
     int16_t sacc;    // accumulator of the special step (-1: none)
     uint16_t pad;
     float coef[4];   // CRY: c.hi c.lo s.hi s.lo
-    uint32_t pad2[4];
+    int16_t acc_x[4]; // accumulators of Im <h|X|v>
+    uint32_t pad2[2];
 };
 static_assert(sizeof(TileStage) == 144, "stage size");
 static_assert(offsetof(TileStage, ry) == 80 && offsetof(TileStage, stab) == 94, "ry .. stab are read as 16 bytes");
+static_assert(offsetof(TileStage, acc_zb) == offsetof(TileStage, acc_y) + 8, "one list of eight");
 
 struct alignas(16) TileRound { // 128 bytes
     uint16_t lo[32]; // byte offset in the tile of lane bits,
@@ -178,7 +180,7 @@ inline bool check_pass(const TilePass &p, int nq, int amp_bytes, int nacc_all) {
         for (int k = 0; k < R[r].nstages; k++) {
             const TileStage &t = S[R[r].stage0 + k];
             for (int i = 0; i < 4; i++)
-                if (t.acc_y[i] >= h.nacc || t.acc_x[i] >= h.nacc) return false;
+                if (t.acc_y[i] >= h.nacc || t.acc_x[i] >= h.nacc || t.acc_zb[i] >= h.nacc) return false;
             if (t.ry >> h.R) return false;
             if ((t.table & 2) && t.tab + (size_t)(1 << h.R) > ntab) return false;
             if ((t.table & 1) && (t.acc_z < 0 || t.acc_z + __builtin_popcount(t.zsel) > h.nacc)) return false;
@@ -1341,7 +1343,7 @@ class Compiler {
         auto reset = [&]() {
             std::memset(&cur, 0, sizeof(cur));
             for (int i = 0; i < 4; i++) {
-                cur.acc_y[i] = cur.acc_x[i] = -1;
+                cur.acc_y[i] = cur.acc_x[i] = cur.acc_zb[i] = -1;
                 turn[i] = nullptr;
             }
             cur.acc_z = cur.sacc = -1;
@@ -1439,6 +1441,11 @@ class Compiler {
                             nacc++;
                         }
                         jac.push_back(JacTerm{z[i].second->slot, acc0 + nacc - 1, z[i].second->coef * scale * scale, z[i].second->ref});
+                    }
+                    if ((cur.zsel & ~0x0116u) == 0) { // masks 1, 2, 4, 8
+                        int next = cur.acc_z;
+                        for (int b = 0; b < 4; b++)
+                            if (cur.zsel >> (1 << b) & 1) cur.acc_zb[b] = (int16_t)next++;
                     }
                 }
                 if (cur.table & 2) last_table_ = Table{pass_, cur.tab, jac0_ + jac.size()};
