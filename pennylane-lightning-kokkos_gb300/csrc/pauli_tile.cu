@@ -88,7 +88,7 @@ struct PauliArgs {
     int nitems, nreal; // the first nreal without a factor i
     int T, ntiles, tiles_x; // tiles_x CTAs walk the tiles, gridDim.x / tiles_x share the items
     int accumulate;
-    int sum_in_df, sum_out_df; // complex128: `out` holds double-float pairs on entry / exit
+    int sum_df; // complex128: `out` holds double-float pairs on exit; what is accumulated to always does
     uint8_t gpos[kPT];      // state bits of the tile, ascending
     uint8_t tpos[kPT];      // those of the thread bits
     uint8_t rpos[kPR];      // and of the register bits
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(kThreads, Ctas<A>::apply) k_pauli_apply_tile(c
         V s[kPA];
         load<A>(a, g, gr, pauli_smem + tl * A::kBytes, true, s);
 #pragma unroll
-        for (int j = 0; j < kPA; j++) s[j] = a.accumulate ? tile::load_amp(a.out, at(g, gr, j), a.sum_in_df, V{}) : V{};
+        for (int j = 0; j < kPA; j++) s[j] = a.accumulate ? tile::load_bits(a.out, at(g, gr, j), V{}) : V{};
         __syncthreads();
 #pragma unroll 1
         for (int k = 0, end; k < a.nitems; k = end) { // up to 16 words, without or with a factor i
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kThreads, Ctas<A>::apply) k_pauli_apply_tile(c
         asm volatile("" : "+r"(go)); // the addresses are formed again, not kept in registers
         __syncthreads(); // partners read before the next tile is loaded
 #pragma unroll
-        for (int j = 0; j < kPA; j++) tile::store_amp(a.out, at(go, gr, j), a.sum_out_df, s[j]);
+        for (int j = 0; j < kPA; j++) tile::store_amp(a.out, at(go, gr, j), a.sum_df, s[j]);
     }
 }
 
@@ -744,6 +744,7 @@ int pauli_tile_expval(plk_state s, const std::vector<PauliGroup> &groups, const 
 
 int pauli_tile_apply(plk_state out, plk_state in, const std::vector<PauliGroup> &groups,
                      const std::vector<PauliTerm> &terms, std::vector<PauliGroup> &rest, bool &accumulate) {
+    accumulate = false;
     // a tile pass reads the state and updates the output; a plain pass gathers
     // 32 patterns from the second-level cache or memory
     if (out->nq < kPT || out->nq > 32 || groups.size() < 2) {
@@ -770,8 +771,7 @@ int pauli_tile_apply(plk_state out, plk_state in, const std::vector<PauliGroup> 
         a.offs = dev.offs;
         a.nitems = pl.item0[i + 1] - pl.item0[i];
         a.accumulate = accumulate;
-        a.sum_in_df = i > 0;
-        a.sum_out_df = i + 1 < pl.passes.size();
+        a.sum_df = i + 1 < pl.passes.size();
         const int grid = std::min(a.ntiles, cap);
         if (c64) k_pauli_apply_tile<AmpC64><<<grid, kThreads, smem, st>>>(a);
         else k_pauli_apply_tile<AmpC128><<<grid, kThreads, smem, st>>>(a);

@@ -32,8 +32,8 @@ struct PauliGroup {
 // their pass) are left in `rest`.  `total` receives the passes' sum.
 int pauli_tile_expval(plk_state s, const std::vector<PauliGroup> &groups, const std::vector<PauliTerm> &terms,
                       std::vector<PauliGroup> &rest, double &total);
-// out = (accumulate ? out : 0) + the taken groups' sum applied to in;
-// accumulate is set once something has been written
+// out = the taken groups' sum applied to in; `accumulate`: whether there were any
+// (else nothing is written)
 int pauli_tile_apply(plk_state out, plk_state in, const std::vector<PauliGroup> &groups,
                      const std::vector<PauliTerm> &terms, std::vector<PauliGroup> &rest, bool &accumulate);
 

@@ -531,15 +531,22 @@ __device__ __forceinline__ DF df_split_near(double x) {
 
 // state buffers: complex128 holds doubles outside a sweep and double-float
 // pairs between its passes
-__device__ __forceinline__ f2x load_amp(const void *p, uint32_t i, int, f2x) {
+__device__ __forceinline__ f2x load_bits(const void *p, uint32_t i, f2x) {
     return __ldcg(static_cast<const unsigned long long *>(p) + i);
 }
-__device__ __forceinline__ AmpC128::V load_amp(const void *p, uint32_t i, int df, AmpC128::V) {
+__device__ __forceinline__ AmpC128::V load_bits(const void *p, uint32_t i, AmpC128::V) {
     const ulonglong2 a = __ldcg(static_cast<const ulonglong2 *>(p) + i);
-    if (df) return {a.x, a.y};
-    const DF re = df_split_near(__longlong_as_double((long long)a.x));
-    const DF im = df_split_near(__longlong_as_double((long long)a.y));
+    return {a.x, a.y};
+}
+__device__ __forceinline__ f2x from_bits(f2x v) { return v; }
+__device__ __forceinline__ AmpC128::V from_bits(const AmpC128::V &v) { // of doubles
+    const DF re = df_split_near(__longlong_as_double((long long)v.h));
+    const DF im = df_split_near(__longlong_as_double((long long)v.l));
     return {f2x_pack(re.hi, im.hi), f2x_pack(re.lo, im.lo)};
+}
+template <class V> __device__ __forceinline__ V load_amp(const void *p, uint32_t i, int df, V) {
+    const V v = load_bits(p, i, V{});
+    return df ? v : from_bits(v);
 }
 // amplitude i of |0...0>
 __device__ __forceinline__ f2x basis_amp(uint32_t i, f2x) { return f2x_pack(i == 0 ? 1.0f : 0.0f, 0.0f); }
@@ -657,19 +664,37 @@ __device__ __forceinline__ void run_tile(const Pass &ps, const Buffers &bf, int 
             const uint32_t g = gev ^ x.lo[lane] ^ x.hi[warp] ^ x.c;
             const uint32_t g0 = x.r[0], g1 = x.r[1], g2 = x.r[2], g3 = x.r[3], g01 = g0 ^ g1, g23 = g2 ^ g3;
             const void *lam = bf.lam_src, *hl = bf.hl;
+            auto at = [&](int j) {
+                return g ^ ((j & 3) == 3 ? g01 : (j & 1) ? g0 : (j & 2) ? g1 : 0u) ^
+                       ((j & 12) == 12 ? g23 : (j & 4) ? g2 : (j & 8) ? g3 : 0u);
+            };
+            // all loads are issued before the first is used
+            if (bf.from_zero) {
 #pragma unroll
-            for (int j = 0; j < NA; j++) {
-                const uint32_t i = g ^ ((j & 3) == 3 ? g01 : (j & 1) ? g0 : (j & 2) ? g1 : 0u) ^
-                                   ((j & 12) == 12 ? g23 : (j & 4) ? g2 : (j & 8) ? g3 : 0u);
-                v[j] = bf.from_zero ? basis_amp(i, V{}) : load_amp(lam, i, bf.in_df, V{});
-                if (BWD) {
-                    if (bf.word) {
-                        const uint32_t k = i ^ bf.wx;
-                        h[j] = load_amp(lam, k, bf.in_df, V{});
+                for (int j = 0; j < NA; j++) v[j] = basis_amp(at(j), V{});
+            } else {
+#pragma unroll
+                for (int j = 0; j < NA; j++) v[j] = load_bits(lam, at(j), V{});
+            }
+            const uint32_t wx = bf.word ? bf.wx : 0u;
+            if (BWD) {
+                const void *from = bf.word ? lam : hl;
+#pragma unroll
+                for (int j = 0; j < NA; j++) h[j] = load_bits(from, at(j) ^ wx, V{});
+            }
+            if (A::kBytes == 16 && !bf.in_df) {
+#pragma unroll
+                for (int j = 0; j < NA; j++) {
+                    if (!bf.from_zero) v[j] = from_bits(v[j]);
+                    if (BWD) h[j] = from_bits(h[j]);
+                }
+            }
+            if (BWD) {
+                if (bf.word) {
+#pragma unroll
+                    for (int j = 0; j < NA; j++) {
                         if (bf.wq & 1u) h[j] = times_i(h[j]);
-                        if ((bf.wq >> 1 ^ __popc(k & bf.wz)) & 1u) h[j] = negate(h[j]);
-                    } else {
-                        h[j] = load_amp(hl, i, bf.in_df, V{});
+                        if ((bf.wq >> 1 ^ __popc((at(j) ^ wx) & bf.wz)) & 1u) h[j] = negate(h[j]);
                     }
                 }
             }
