@@ -10,7 +10,7 @@
 // of up to 11 qubits is one CTA's work per pass.  States live in one buffer, in
 // waves of circuits when they are too large together.
 //
-// 128 circuits of 8-20 qubits, 5-30 layers on one GB300: 105.3 -> 16.0 ms a run
+// 128 circuits of 8-20 qubits, 5-30 layers on one GB300: 105.3 -> 15.3 ms a run
 // (the engine's register windows spilled, and its largest circuits streamed their
 // states from memory at 15 % of its bandwidth, one 8-CTA cluster each), first run
 // with compilation 142 -> 39 ms.
@@ -45,6 +45,7 @@ struct Job { // one pass of one circuit
     uint32_t prog_bytes;
     int32_t T, nacc;
     int32_t first_pass;   // forward: starts from |0...0>
+    int32_t last_pass;    // backward: leaves no states
     uint64_t part;        // partial sums: [accumulator][CTA]
     int32_t nctas;
 };
@@ -281,7 +282,7 @@ __global__ void __launch_bounds__(kBThreads, BWD ? kBCtasBwd : kBCtasFwd)
         for (int i = lane; i < j.nacc; i += 32) row[i] = make_float2(0.0f, 0.0f);
     __syncthreads();
     const Pass ps(prog);
-    const Buffers bf{states + j.lam, states + j.lam, states + j.hl, 0, 0, !BWD && j.first_pass, false, 0, 0, 0};
+    const Buffers bf{states + j.lam, states + j.lam, states + j.hl, 0, 0, !BWD && j.first_pass, BWD && j.last_pass, false, 0, 0, 0};
     for (int t = 0; t < c.ntiles; t++) run_tile<AmpC64, kBR, BWD>(ps, bf, c.tile0 + t, j.T, L, M, row);
     if (BWD) {
         for (int i = tid; i < j.nacc; i += blockDim.x) {
@@ -733,6 +734,7 @@ int build(BatchTiles *t, const std::vector<BatchCircuit> &circs, const BasisTabl
                     j.T = P.T;
                     j.nacc = h.nacc;
                     j.first_pass = p == 0;
+                    j.last_pass = p + 1 == (int)P.passes.size();
                     j.nctas = (ntiles + each - 1) / each;
                     j.part = npart;
                     npart += (uint64_t)h.nacc * j.nctas;

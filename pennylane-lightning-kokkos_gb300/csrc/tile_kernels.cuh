@@ -49,6 +49,7 @@ struct Args {
     int T, nacc, ntiles;
     int nacc_all;      // accumulators of the whole program
     int in_df, out_df; // complex128: buffers hold double-float pairs on entry / exit
+    int drop;          // the states on exit are not wanted
     double *part;      // [sweep][accumulator][gridDim.x]
     // when set, H lambda of sweep y starts as the Pauli word i^ny (-1)^popcount(k & z) |k ^ x> on lam_src[y]
     int words;
@@ -617,6 +618,8 @@ struct Buffers {
     void *lam, *hl;
     int in_df, out_df; // complex128: double-float pairs on entry / exit
     bool from_zero;    // the state is |0...0> on entry, lam_src is not read
+    bool drop;         // the states on exit are not written: a backward sweep's last pass on buffers of its own
+                       // (Jacobian of 20 observables on 20 qubits complex128 30.21 -> 30.06 ms)
     bool word;         // H lambda is a Pauli word on lam_src, hl is not read
     uint32_t wx, wz, wq;
 };
@@ -786,7 +789,7 @@ __device__ __forceinline__ void run_tile(const Pass &ps, const Buffers &bf, int 
                 A::st(L + slot(j), v[j]);
                 if (BWD) A::st(M + slot(j), h[j]);
             }
-        } else {
+        } else if (!BWD || !bf.drop) {
             if (nrounds == 1) __syncthreads(); // all of the tile read before any of it is written
             uint32_t go = base;
             for (int k = hd.ev_store0; k < hd.nev; k++)
@@ -822,7 +825,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_tile(const __grid_constant__ 
         for (int i = lane; i < a.nacc; i += 32) row[i] = make_float2(0.0f, 0.0f);
     __syncthreads();
     const Pass ps(prog);
-    const Buffers bf{a.lam_src[blockIdx.y], a.lam[blockIdx.y], a.hl[blockIdx.y], a.in_df, a.out_df, false,
+    const Buffers bf{a.lam_src[blockIdx.y], a.lam[blockIdx.y], a.hl[blockIdx.y], a.in_df, a.out_df, false, BWD && a.drop,
                      BWD && a.words, a.wx[blockIdx.y], a.wz[blockIdx.y], a.wq[blockIdx.y]};
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) run_tile<A, R, BWD>(ps, bf, tile, a.T, L, M, row);
     if (BWD) {
