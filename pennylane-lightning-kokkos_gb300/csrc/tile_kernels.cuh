@@ -557,8 +557,15 @@ __device__ __forceinline__ AmpC128::V basis_amp(uint32_t i, AmpC128::V) {
 __device__ __forceinline__ void store_amp(void *p, uint32_t i, int, f2x v) {
     __stcg(static_cast<unsigned long long *>(p) + i, v);
 }
+// Between passes the high and low parts are set apart again: rotations leave the
+// low part unnormalised, it collects rounding errors and is itself rounded at
+// their size (state errors over a list of gates: 1.9e-13 without, 6e-14 with).
 __device__ __forceinline__ void store_amp(void *p, uint32_t i, int df, AmpC128::V v) {
-    if (!df) {
+    if (df) {
+        const f2x s = f2x_add(v.h, v.l);
+        v.l = f2x_sub(v.l, f2x_sub(s, v.h));
+        v.h = s;
+    } else {
         const double re = df_join(f2x_lo(v.h), f2x_lo(v.l)), im = df_join(f2x_hi(v.h), f2x_hi(v.l));
         v = {(f2x)__double_as_longlong(re), (f2x)__double_as_longlong(im)};
     }
