@@ -259,12 +259,14 @@ PLK_API int plk_adjoint_jacobian_pauli(plk_state lambda, int32_t num_obs, const 
 PLK_API int plk_expval_pauliz_noalloc(const void *state, int32_t num_qubits, int32_t dtype, int32_t count,
                                       const int64_t *wires, double *out, void *cuda_stream);
 
-/* ---- register-window path ----------------------------------------------- */
-/* Op lists (plk_apply_ops) and adjoint Jacobians run as register-window
- * sweeps (about seven ops per state pass; complex128 in double-float on the
- * FP32 pipe; with several observables one backward sweep per observable on
- * a copy of lambda, when that moves fewer bytes) unless this is switched
- * off; results agree with the op-at-a-time path to rounding. */
+/* ---- sweep path ---------------------------------------------------------- */
+/* Op lists (plk_apply_ops) and adjoint Jacobians run as sweeps that apply many
+ * ops per state pass unless this is switched off: as tile programs (passes
+ * over shared-memory tiles of 2^11 to 2^12 amplitudes), or, with dense
+ * matrices in the list, as register windows of four bits; complex128 in
+ * double-float on the FP32 pipe; with several observables one backward sweep
+ * per observable on a copy of lambda, when that moves fewer bytes.  Results
+ * agree with the op-at-a-time path to rounding. */
 PLK_API int plk_set_window_path(int32_t enable);
 PLK_API int plk_get_window_path(int32_t *enabled);
 
@@ -304,8 +306,9 @@ PLK_API int plk_gate_matrix(int32_t gate, const double *params, int32_t num_para
 /* Many independent circuits (own qubit count 4..30, own gates and
  * parameters, own Pauli-sum observable) evaluated together: for every circuit
  * the forward pass from |0...0>, <H> and the adjoint gradient d<H>/dtheta of
- * its trainable parameters, in one persistent launch (replayed as a CUDA
- * graph).  Per circuit this is what the reference's device does one tape at
+ * its trainable parameters, in a fixed sequence of launches (replayed as a CUDA
+ * graph; complex128 batches and batches with dense matrices in one persistent
+ * launch).  Per circuit this is what the reference's device does one tape at
  * a time: apply the tape (StateVectorKokkos::applyOperation,
  * StateVectorKokkos.hpp:585-676), the Hamiltonian expectation
  * (ObservablesKokkos.hpp:484-494) and AdjointJacobianKokkos::adjointJacobian

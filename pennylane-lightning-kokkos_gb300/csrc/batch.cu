@@ -12,6 +12,9 @@
 // The reference runs this one circuit at a time (the Python device loops over
 // tapes); here a batch is compiled once into register windows and a CUDA
 // graph replays [parameters H2D, matrix preparation, engine, results D2H].
+// complex64 batches without dense matrices run on tiles instead (batch_tile.cu:
+// 128 circuits of 8-20 qubits 105 ms a run here, 15.3 there); what follows is for
+// the others.
 //
 // Gate matrices come from the same gate plans as the per-state kernels
 // (plan_gate / plan_generator), expanded to dense matrices on the host.  A

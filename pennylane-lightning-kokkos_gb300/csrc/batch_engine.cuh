@@ -1,4 +1,5 @@
-// batch_engine.cuh — device side of the batched-circuit engine.
+// batch_engine.cuh — device side of the batched-circuit engine, for complex128
+// batches and batches with dense matrices (complex64 without them: batch_tile.cu).
 //
 // Many independent circuits (each with its own qubit count, gates, parameters
 // and Pauli-sum observable) run forward, <H> and the adjoint gradient in one

@@ -1,7 +1,8 @@
 // window_host.cuh — host side of the register-window engine: dense gate
 // matrices from the gate plans, their trigonometric fit in the parameter,
 // expanded ops, and the compiler that packs an op sequence into 4-qubit
-// register windows (used for batches and for single large states).
+// register windows (used for batches of complex128 circuits or with dense
+// matrices, and for single states under op lists with dense matrices).
 #pragma once
 
 #include <algorithm>

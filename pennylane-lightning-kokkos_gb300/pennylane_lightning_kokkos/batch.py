@@ -1,8 +1,8 @@
 """Batches of independent circuits: forward, <H> and adjoint gradient together.
 
 ``CircuitBatch`` collects circuits, each with its own qubit count, gate list,
-parameters and Pauli-sum observable, and evaluates all of them in one
-persistent GPU launch replayed as a CUDA graph (``plk_batch_*`` in the C ABI).
+parameters and Pauli-sum observable, and evaluates all of them in a fixed
+sequence of GPU launches replayed as a CUDA graph (``plk_batch_*`` in the C ABI).
 For every circuit it returns what the reference device computes per tape:
 the expectation value of the observable after the circuit
 (``LightningKokkos.expval``, lightning_kokkos.py:403-430) and its adjoint

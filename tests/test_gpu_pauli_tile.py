@@ -80,3 +80,30 @@ def test_pauli_sum(nq, kind, dtype):
     np.testing.assert_allclose(o.get(), ref, atol=TOL[dtype] * scale, rtol=0)
     s.close()
     o.close()
+
+
+@pytest.mark.parametrize("nq", [9, 13, 16])
+def test_cancelling_energy_keeps_low_bits(nq):
+    """complex128 energies of many words whose terms cancel, on a state with a few
+    large amplitudes.  Coefficients carry 48 bits (2^-49 each), products 2^-48,
+    sums are settled after each word: within 2^-46 of the sum of |coefficients|."""
+    rng = np.random.default_rng(7 * nq)
+    psi = np.ones(1)
+    for a in rng.uniform(0.2, 0.6, nq): # product state, probabilities over many decades
+        psi = np.kron(psi, [np.cos(a), np.sin(a) * np.exp(1j * a)])
+    words = []
+    for _ in range(60):
+        wt = int(rng.integers(1, 5))
+        wires = [int(w) for w in rng.choice(nq, wt, replace=False)]
+        letters = "".join(str(x) for x in rng.choice(list("XYZ"), wt))
+        c = float(rng.standard_normal())
+        words += [(c, wires, letters), (-c * (1 + 1e-9), wires, letters)]
+    s = State.from_array(psi, N.PLK_C128)
+    want = sum(float(np.vdot(psi, dense(psi, nq, [w])).real) for w in words)
+    c, cp = f64([w[0] for w in words])
+    off, offp = i64(np.cumsum([0] + [len(w[1]) for w in words]))
+    wi, wp = i64([x for w in words for x in w[1]])
+    v = C.c_double()
+    N.check(N.lib.plk_expval_pauli_sum(s.h, len(words), cp, offp, wp, "".join(w[2] for w in words).encode(), C.byref(v)))
+    assert abs(v.value - want) < 2.0**-46 * float(np.sum(np.abs(c)))
+    s.close()
