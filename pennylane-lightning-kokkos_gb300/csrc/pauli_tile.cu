@@ -582,6 +582,45 @@ uint32_t choose_register_bits(const Pass &p, int nq, int T, int low, const std::
     return reg;
 }
 
+// Application: which passes are worth it.  A tile pass reads the state and updates
+// the output for its words; the plain kernel does that once for 32 patterns and
+// gathers each pattern's source.  Costs per tile pass, per word in it, per plain
+// pass and per word in that are times at 24 qubits in us: 40 words of weight 8
+// complex64, some four to a tile pass, 989 on tiles and 605 in plain passes; 40 words
+// of weight 4 450 and 596; complex128 1915 and 2406, 1190 and 2356.
+void keep_worthwhile(bool c64, const std::vector<PauliGroup> &groups, std::vector<Pass> &passes,
+                     std::vector<PauliGroup> &rest) {
+    struct Cost {
+        double pass, word, plain, plain_word;
+    };
+    const Cost c = c64 ? Cost{52, 6.5, 30, 14.5} : Cost{115, 22, 100, 57};
+    auto words = [&](const Pass &p) {
+        int n = 0;
+        for (int gi : p.groups) n += groups[gi].count;
+        return n;
+    };
+    std::stable_sort(passes.begin(), passes.end(), [&](const Pass &x, const Pass &y) { return words(x) > words(y); });
+    // the passes with most words on tiles, the others plain: the cheapest split
+    size_t best = passes.size(), left = rest.size();
+    double least = 0.0, plain = 0.0, on_tiles = 0.0;
+    for (const Pass &p : passes) on_tiles += c.pass + c.word * words(p);
+    for (size_t k = passes.size() + 1; k-- > 0;) {
+        if (k < passes.size()) {
+            on_tiles -= c.pass + c.word * words(passes[k]);
+            plain += c.plain_word * words(passes[k]);
+            left += passes[k].groups.size();
+        }
+        const double cost = on_tiles + plain + c.plain * (double)((left + 31) / 32);
+        if (k == passes.size() || cost < least) {
+            least = cost;
+            best = k;
+        }
+    }
+    for (size_t k = best; k < passes.size(); k++)
+        for (int gi : passes[k].groups) rest.push_back(groups[gi]);
+    passes.resize(best);
+}
+
 // expval: Hermitian form, each pair once
 void make_plan(int nq, int dtype, const std::vector<PauliGroup> &groups, const std::vector<PauliTerm> &terms,
                bool expval, Plan &pl, std::vector<PauliGroup> &rest) {
@@ -590,6 +629,7 @@ void make_plan(int nq, int dtype, const std::vector<PauliGroup> &groups, const s
     const int low = std::min(c64 ? 3 : 2, T);
     const int least = expval ? (c64 ? kManyExpvalC64 : kManyExpvalC128) : (c64 ? kManyApplyC64 : kManyApplyC128);
     choose_passes(nq, T, low, groups, pl.passes, rest);
+    if (!expval) keep_worthwhile(c64, groups, pl.passes, rest);
     for (const Pass &p : pl.passes) {
         PauliArgs a;
         std::memset((void *)&a, 0, sizeof(a));
@@ -747,7 +787,10 @@ int pauli_tile_apply(plk_state out, plk_state in, const std::vector<PauliGroup> 
     accumulate = false;
     // a tile pass reads the state and updates the output; a plain pass gathers
     // 32 patterns from the second-level cache or memory
-    if (out->nq < kPT || out->nq > 32 || groups.size() < 2) {
+    // (on small states a launch costs more than its words: 40 words of weight 8, us on
+    // tiles / plain, 13 qubits complex64 49 / 40 and complex128 67 / 73, 16 qubits
+    // 44 / 40 and 85 / 76)
+    if (out->nq < 18 || out->nq > 32 || groups.size() < 2) {
         rest = groups;
         return PLK_OK;
     }

@@ -107,3 +107,33 @@ def test_cancelling_energy_keeps_low_bits(nq):
     N.check(N.lib.plk_expval_pauli_sum(s.h, len(words), cp, offp, wp, "".join(w[2] for w in words).encode(), C.byref(v)))
     assert abs(v.value - want) < 2.0**-46 * float(np.sum(np.abs(c)))
     s.close()
+
+
+@pytest.mark.parametrize("dtype", [N.PLK_C64, N.PLK_C128])
+@pytest.mark.parametrize("wt", [2, 7])
+def test_application_splits_between_tiles_and_plain_passes(wt, dtype):
+    """Narrow words go to tiles, wide ones to the plain kernel, some sums to both
+    (18 qubits, the smallest state whose applications use tiles)."""
+    nq, rng = 18, np.random.default_rng(wt)
+    psi = rand_state(nq, rng)
+    words = []
+    for k in range(40):
+        w = wt if k % 2 else 1
+        words.append((float(rng.standard_normal()), [int(x) for x in rng.choice(nq, w, replace=False)],
+                      "".join(str(x) for x in rng.choice(list("XYZ"), w))))
+    s, o = State.from_array(psi, dtype), State(nq, dtype)
+    idx = np.arange(1 << nq)
+    par = np.array([bin(k).count("1") & 1 for k in range(1 << 9)])
+    have, ref = s.get().astype(np.complex128), np.zeros(1 << nq, dtype=np.complex128)
+    for c, wires, letters in words:
+        x = sum(1 << (nq - 1 - w) for w, l in zip(wires, letters) if l in "XY")
+        z = sum(1 << (nq - 1 - w) for w, l in zip(wires, letters) if l in "YZ")
+        t = (idx ^ x) & z
+        ref += c * 1j ** letters.count("Y") * (1 - 2 * (par[t & 511] ^ par[t >> 9])) * have[idx ^ x]
+    c, cp = f64([w[0] for w in words])
+    off, offp = i64(np.cumsum([0] + [len(w[1]) for w in words]))
+    wi, wp = i64([x for w in words for x in w[1]])
+    N.check(N.lib.plk_apply_pauli_sum(o.h, s.h, len(words), cp, offp, wp, "".join(w[2] for w in words).encode()))
+    np.testing.assert_allclose(o.get(), ref, atol=TOL[dtype] * float(np.sum(np.abs(c))), rtol=0)
+    s.close()
+    o.close()
