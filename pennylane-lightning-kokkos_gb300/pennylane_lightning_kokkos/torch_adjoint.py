@@ -109,12 +109,14 @@ class AdjointCircuit:
             self.ops.append((g, wires, inv, k if npar == 1 else -1))
             k += npar
         self.num_params = k
-        # the tape as one array of PlkOp records; a call adds its parameters
-        # (built op by op through ctypes a tape took 5 us per op, a tenth of a
-        # 26-qubit gradient and most of a small one)
+        # the tape as one array of PlkOp records; a call adds the addresses of
+        # its wires and parameters, never kept here: a copied or unpickled
+        # circuit has arrays of its own (built op by op through ctypes a tape
+        # took 5 us per op, a tenth of a 26-qubit gradient and most of a small one)
         n = len(self.ops)
         counts = np.array([len(w) for _, w, _, _ in self.ops], dtype=np.int64)
-        starts = np.concatenate([[0], np.cumsum(counts)[:-1]]) if n else counts
+        self._wires_at = np.zeros(max(1, n), dtype=np.uint64) # byte offsets of the ops' wires
+        self._wires_at[1:n] = 8 * np.cumsum(counts)[:-1]
         self._wires = np.array([x for _, w, _, _ in self.ops for x in w] or [0], dtype=np.int64)
         self._param_of = np.array([pi for _, _, _, pi in self.ops], dtype=np.int64)
         self._records = np.zeros(max(1, n), dtype=np.dtype(
@@ -124,7 +126,6 @@ class AdjointCircuit:
             self._records["nw"] = counts
             self._records["adj"] = [int(inv) for _, _, inv, _ in self.ops]
             self._records["np"] = self._param_of >= 0
-            self._records["w"] = self._wires.ctypes.data + 8 * starts.astype(np.uint64)
         self._trainable = np.flatnonzero(self._param_of >= 0)
 
     # -- helpers -----------------------------------------------------------
@@ -134,8 +135,9 @@ class AdjointCircuit:
         if len(self._trainable):
             values[self._trainable] = params[self._param_of[self._trainable]]
         records = self._records.copy()
+        records["w"] = self._wires.ctypes.data + self._wires_at
         records["p"] = values.ctypes.data + 8 * np.arange(len(records), dtype=np.uint64)
-        return C.cast(records.ctypes.data, C.POINTER(N.PlkOp)), (records, values)
+        return C.cast(records.ctypes.data, C.POINTER(N.PlkOp)), (records, self._wires, values)
 
     def _stream(self):
         return torch.cuda.current_stream(self.device).cuda_stream
