@@ -1377,6 +1377,21 @@ class Compiler {
             if (any) o.stages.push_back(cur);
             reset();
         };
+        // A stage that begins without a table gets one when the sweep holds more
+        // than 2^8 times the state.  A stage turns at most kMaxRegBits bits by at
+        // most sqrt(2) each, so what is held stays within 2^10, and a sum's
+        // products within 2^20: controlled rotations between rotations, which meet
+        // no phase, reached 2^64 and 2^128 when this was looked at once per round.
+        auto begin = [&]() {
+            if (!any && pend_ < 1.0 / 256) {
+                cur.table |= 2;
+                cur.tab = (uint16_t)tab_pos(o);
+                for (int j = 0; j < amps; j++) put(o, pend_);
+                pend_ = 1;
+                last_table_ = Table{pass_, cur.tab, jac0_ + jac.size()};
+            }
+            any = true;
+        };
         reset();
         std::vector<std::pair<uint32_t, const ZTerm *>> z;
         for (const Step &s : st) {
@@ -1452,12 +1467,12 @@ class Compiler {
             } else if (s.kind == SK_RY) {
                 const int b = reg_of(s.u->p.t);
                 if (cur.special || turn[b]) flush();
-                any = true;
+                begin();
                 turn[b] = s.u;
             } else {
                 if (cur.special) flush();
                 turns();
-                any = true;
+                begin();
                 const Unit &u = *s.u;
                 if (s.kind == SK_CRY) {
                     cur.special = TS_CRY;
@@ -1606,14 +1621,6 @@ class Compiler {
                 place(st, u, regs);
             }
             for (int k = T_ - 1; k >= 0 && popc(regs) < R_; k--) regs |= 1u << o.tbits[k];
-            if (pend_ < 1.0 / 256) { // keep what the sweep holds within 2^12 of the state
-                bool table = false;
-                for (const Step &x : st) table = table || x.kind == SK_TAB;
-                if (!table) {
-                    st.insert(st.begin(), Step{});
-                    st.front().kind = SK_TAB;
-                }
-            }
             ok = !st.empty() && emit_round(o, st, regs, acc0, jac, nacc);
         }
         for (int i : sel) in_[i] = 0, deg_[i] = 0;
