@@ -278,7 +278,11 @@ PLK_API int plk_get_window_path(int32_t *enabled);
  * 2^-45 relative error per gate; values below about 2^-103 lose their low
  * part and below 2^-126 become zero), because this GPU's FP64 pipe is about
  * 1/64 of its FP32 rate.  PLK_ARITH_FP64: native IEEE double arithmetic (and
- * no register-window sweeps), slower for dense matrices and rotations.  The
+ * no tile or register-window sweeps), slower for dense matrices and rotations.
+ * Expectation values of named observables, matrices and Pauli sums, applied
+ * Pauli sums and inner products work in double-float in both modes; but in FP64
+ * mode the pair products of a Pauli word that shares its X pattern with no other
+ * word of an expectation value are formed in FP64.  The
  * environment variable PLK_C128_ARITH=fp64 selects the initial mode; the
  * setting applies to calls made after it. */
 enum { PLK_ARITH_DOUBLE_FLOAT = 0, PLK_ARITH_FP64 = 1 };

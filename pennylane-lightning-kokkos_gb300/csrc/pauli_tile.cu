@@ -730,6 +730,11 @@ int upload(const Plan &pl, int device, cudaStream_t st, PoolBuf &buf, PauliArgs 
 // the slots of a small tile are as far apart as a large one's
 size_t smem_of(int dtype) { return (size_t)(dtype == PLK_C64 ? 8 : 16) << kPT; }
 
+// Tiles hold double-float pairs: complex128 with native FP64 arithmetic asked for
+// keeps the kernels of expval.cu, whose one-word products are formed in FP64
+// (amplitudes of 2^150 and 2^-150 read as 0 here and multiply to 1 there).
+bool tiles_allowed(int dtype) { return dtype == PLK_C64 || c128_use_df(); }
+
 template <class K> int opt_in(K kernel, size_t bytes) {
     if (bytes > 48 * 1024) PLK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     return PLK_OK;
@@ -740,7 +745,7 @@ template <class K> int opt_in(K kernel, size_t bytes) {
 int pauli_tile_expval(plk_state s, const std::vector<PauliGroup> &groups, const std::vector<PauliTerm> &terms,
                       std::vector<PauliGroup> &rest, double &total) {
     total = 0.0;
-    if (s->nq < kPR || s->nq > 32 || groups.size() < 2) {
+    if (s->nq < kPR || s->nq > 32 || groups.size() < 2 || !tiles_allowed(s->dtype)) {
         rest = groups;
         return PLK_OK;
     }
@@ -790,7 +795,7 @@ int pauli_tile_apply(plk_state out, plk_state in, const std::vector<PauliGroup> 
     // (on small states a launch costs more than its words: 40 words of weight 8, us on
     // tiles / plain, 13 qubits complex64 49 / 40 and complex128 67 / 73, 16 qubits
     // 44 / 40 and 85 / 76)
-    if (out->nq < 18 || out->nq > 32 || groups.size() < 2) {
+    if (out->nq < 18 || out->nq > 32 || groups.size() < 2 || !tiles_allowed(out->dtype)) {
         rest = groups;
         return PLK_OK;
     }
