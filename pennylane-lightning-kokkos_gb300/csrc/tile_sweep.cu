@@ -363,12 +363,14 @@ PLK_API int plk_adjoint_jacobian_pauli(plk_state lambda, int32_t num_obs, const 
     PLK_TRY(adjoint_checks(lambda, nullptr, 0, ops, num_ops, trainable, num_trainable, jac));
     if (num_obs < 1 || !coeffs || !offsets) PLK_FAIL(PLK_ERR_INVALID_ARG, "bad Pauli-word arguments");
     PLK_CUDA(cudaSetDevice(lambda->device));
+    if (lambda->nq > 32) PLK_FAIL(PLK_ERR_UNSUPPORTED, "this state's sweeps do not start from Pauli words");
     std::vector<tile::Word> words;
     for (int o = 0; o < num_obs; o++) {
         tile::Word w{0, 0, 0, coeffs[o]};
+        if (offsets[o + 1] < offsets[o]) PLK_FAIL(PLK_ERR_INVALID_ARG, "Pauli-word offsets must be non-decreasing");
         for (int64_t j = offsets[o]; j < offsets[o + 1]; j++) {
-            if (!wires || !paulis || wires[j] < 0 || wires[j] >= lambda->nq || lambda->nq > 32)
-                PLK_FAIL(PLK_ERR_INVALID_ARG, "Pauli word wire out of range");
+            if (!wires || !paulis) PLK_FAIL(PLK_ERR_INVALID_ARG, "bad Pauli-word arguments");
+            if (wires[j] < 0 || wires[j] >= lambda->nq) PLK_FAIL(PLK_ERR_INVALID_ARG, "Pauli word wire out of range");
             const uint32_t bit = 1u << (lambda->nq - 1 - wires[j]);
             if ((w.x | w.z) & bit) PLK_FAIL(PLK_ERR_INVALID_ARG, "repeated wire in a Pauli word");
             switch (paulis[j]) {
