@@ -37,8 +37,8 @@ Printed JSON line:
                FP64 accumulation vs complex128, seconds per gradient and the
                largest gradient difference
   batch      - 4096 circuits (8-20 qubits, 5-30 layers, 10-term Hamiltonians),
-               forward + <H> + adjoint gradient in one persistent complex64
-               launch replayed as a CUDA graph (autotuned), circuits/s,
+               forward + <H> + adjoint gradient in complex64 as tile programs
+               of all circuits together, one CUDA graph, circuits/s,
                against a per-circuit loop of the plain path and the oracle
   plain_20q  - 20-qubit complex128 circuit (600 parameters), 20 <PauliZ> and
                the 20 x 600 Jacobian through the reference-facing module,
@@ -98,7 +98,7 @@ def parse_args(argv=None):
     ap.add_argument("--only", choices=["adjoint", "batch", "plain20", "precision", "kernels", "parity"],
                     default=None, help="run one secondary config alone and print its JSON (profiling, spot checks, "
                                        "and the full-size oracle parity run)")
-    ap.add_argument("--no-tune", action="store_true", help="batch: fixed launch configuration instead of autotuning")
+    ap.add_argument("--no-tune", action="store_true", help="batch: accepted, no effect (tile programs have no launch configuration)")
     ap.add_argument("--no-precision", action="store_true",
                     help="skip the equal-bytes precision config (32-qubit complex64 vs 31-qubit complex128)")
     ap.add_argument("--no-fp64", action="store_true", help="skip the native-FP64 pass of the gate sweep")
@@ -736,8 +736,8 @@ def plain_circuit_gradient(m, bits, device, nq, ops, words):
 
 def run_batch(args, device, torch):
     """Batching: forward + <H> + adjoint gradient of every circuit of a
-    seeded uneven batch in one persistent complex64 launch (CUDA graph),
-    against a per-circuit loop of the plain path and the oracle."""
+    seeded uneven batch in complex64, tile programs of all circuits together
+    (CUDA graph), against a per-circuit loop of the plain path and the oracle."""
     import pennylane_lightning_kokkos.lightning_kokkos_qubit_ops as m
     from pennylane_lightning_kokkos.batch import CircuitBatch
     from pennylane_lightning_kokkos.circuits import batch_workload_packed, packed_to_ops
@@ -746,24 +746,9 @@ def run_batch(args, device, torch):
     wl = batch_workload_packed(n, seed=5)
     work = np.array([len(pk["gates"]) * float(1 << nq) for nq, pk, _ in wl])
     gate_apps = sum(len(pk["gates"]) for _, pk, _ in wl)
-    # autotune on a one-in-sixteen subsample, then run the whole batch with the winner
-    if args.no_tune:
-        report, tune_s = "not tuned", 0.0
-        cfg = {"cluster": 8, "smem_qubits": 12, "cluster_min_qubits": 13, "ctas_per_sm": 2}
-    else:
-        sub = CircuitBatch("c64", device)
-        for nq, pk, words in wl[::16]:
-            sub.add_packed(nq, pk, words)
-        t = time.perf_counter()
-        report = sub.tune(reps=1)
-        tune_s = time.perf_counter() - t
-        cfg = sub.get_config()
-        sub.close()
     b = CircuitBatch("c64", device)
     for nq, pk, words in wl:
         b.add_packed(nq, pk, words)
-    b.set_config(cluster=cfg["cluster"], smem_qubits=cfg["smem_qubits"], cluster_min_qubits=cfg["cluster_min_qubits"],
-                 ctas_per_sm=cfg["ctas_per_sm"])
     t = time.perf_counter()
     b.run()
     first_s = time.perf_counter() - t
@@ -783,12 +768,11 @@ def run_batch(args, device, torch):
     out = {"circuits": n, "qubits": "uniform 8-20", "layers": "uniform 5-30 (RX, RY, RZ + CNOT ladder)",
            "hamiltonian_terms": 10, "dtype": "complex64 state, double-float accumulation",
            "params": int(npar), "gate_applications_forward": int(gate_apps),
-           "tuned_config": cfg, "tune_seconds": tune_s, "first_run_seconds": first_s,
+           "first_run_seconds": first_s,
            "device_ms": ms, "circuits_per_s": n / (ms / 1e3),
            "e2e_circuits_per_s": n / statistics.median(wall_s),
            "e2e_api": "CircuitBatch.run (parameters in, <H> and gradients out, host arrays)",
-           "gate_applications_per_s": gate_apps / (ms / 1e3), "kernel_launches_per_run": int(launches),
-           "tune_report": report.strip().splitlines()}
+           "gate_applications_per_s": gate_apps / (ms / 1e3), "kernel_launches_per_run": int(launches)}
     # accuracy: complex128 batch on a sample
     idx = list(range(0, n, max(1, n // 64)))
     b128 = CircuitBatch("c128", device)

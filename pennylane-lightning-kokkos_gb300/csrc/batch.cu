@@ -588,8 +588,8 @@ template <class T, int NT, int MINB> static int launch_engine(plk_batch b, const
 static int cfg_key(const BatchConfig &c) {
     return (((c.cluster * 4 + c.ctas_per_sm) * 1024 + c.threads) * 64 + c.smem_bits) * 64 + c.cluster_min_qubits;
 }
-
-
+// what a captured graph depends on: the engine's configuration, which tiles have none of
+static int graph_key(plk_batch b) { return b->tiles ? 0 : cfg_key(b->cfg); }
 
 template <class T> static int prepare_run(plk_batch b) {
     if (!b->compiled) {
@@ -660,7 +660,7 @@ template <class T> static int run_host(plk_batch b, double *expval, double *jac)
     const size_t npar = b->params.size();
     cudaStream_t st = b->stream;
     std::memcpy(b->h_params_pinned, b->params.data(), npar * sizeof(double));
-    if (b->use_graph && b->graph_cfg_key != cfg_key(b->cfg)) {
+    if (b->use_graph && b->graph_cfg_key != graph_key(b)) {
         if (b->graph) cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
         cudaGraph_t g = nullptr;
@@ -687,7 +687,7 @@ template <class T> static int run_host(plk_batch b, double *expval, double *jac)
         const cudaError_t ei = cudaGraphInstantiate(&b->graph, g, 0);
         cudaGraphDestroy(g);
         PLK_CUDA(ei);
-        b->graph_cfg_key = cfg_key(b->cfg);
+        b->graph_cfg_key = graph_key(b);
     }
     cudaEvent_t e0, e1;
     PLK_CUDA(cudaEventCreate(&e0));
@@ -1055,12 +1055,39 @@ PLK_API int plk_batch_last_time(plk_batch b, double *ms, int64_t *launches) {
 }
 
 // Autotuner: times every configuration of a small grid on this batch and
-// keeps the fastest (median of `reps` graph replays after one warm-up).
+// keeps the fastest (median of `reps` graph replays after one warm-up).  Tile
+// programs have no configuration: one time is reported and none is chosen.
 PLK_API int plk_batch_tune(plk_batch b, int32_t reps, char *report, int32_t report_len) {
     if (!b) PLK_FAIL(PLK_ERR_INVALID_ARG, "null batch");
     if (b->circs.empty()) PLK_FAIL(PLK_ERR_INVALID_ARG, "empty batch");
     PLK_CUDA(cudaSetDevice(b->device));
     reps = std::max(1, reps);
+    auto timed = [&](double &ms) -> int { // median of `reps` runs
+        std::vector<double> t;
+        for (int r = 0; r < reps; r++) {
+            PLK_TRY(plk_batch_run(b, nullptr, nullptr));
+            t.push_back(b->last_ms);
+        }
+        std::sort(t.begin(), t.end());
+        ms = t[t.size() / 2];
+        return PLK_OK;
+    };
+    auto give = [&](const std::string &rep) {
+        if (report && report_len > 0) {
+            std::strncpy(report, rep.c_str(), (size_t)report_len - 1);
+            report[report_len - 1] = 0;
+        }
+    };
+    if (b->dtype == PLK_C64 && !b->compiled) prepare_run<float>(b); // a configuration that fails is met below
+    if (b->tiles) {
+        double ms = 0.0;
+        PLK_TRY(plk_batch_run(b, nullptr, nullptr)); // warm-up
+        PLK_TRY(timed(ms));
+        char line[96];
+        std::snprintf(line, sizeof(line), "tile programs, nothing to tune: %.3f ms\n", ms);
+        give(line);
+        return PLK_OK;
+    }
     const BatchConfig saved = b->cfg;
     std::vector<BatchConfig> cands;
     int max_nq = 0;
@@ -1093,13 +1120,8 @@ PLK_API int plk_batch_tune(plk_batch b, int32_t reps, char *report, int32_t repo
                    " cluster_min=" + std::to_string(c.cluster_min_qubits) + " failed: " + last_error() + "\n";
             continue;
         }
-        std::vector<double> t;
-        for (int r = 0; r < reps; r++) {
-            PLK_TRY(plk_batch_run(b, nullptr, nullptr));
-            t.push_back(b->last_ms);
-        }
-        std::sort(t.begin(), t.end());
-        const double med = t[t.size() / 2];
+        double med = 0.0;
+        PLK_TRY(timed(med));
         char line[160];
         std::snprintf(line, sizeof(line), "ctas_per_sm=%d cluster=%d smem_qubits=%d cluster_min=%d: %.3f ms\n",
                       c.ctas_per_sm, c.cluster, c.smem_bits, c.cluster_min_qubits, med);
@@ -1111,10 +1133,7 @@ PLK_API int plk_batch_tune(plk_batch b, int32_t reps, char *report, int32_t repo
     }
     b->cfg = best_cfg;
     b->tuned = true;
-    if (report && report_len > 0) {
-        std::strncpy(report, rep.c_str(), (size_t)report_len - 1);
-        report[report_len - 1] = 0;
-    }
+    give(rep);
     return PLK_OK;
 }
 

@@ -158,6 +158,8 @@ class CircuitBatch:
         N.check(N.lib.plk_batch_set_graph(self._h, int(use)))
 
     def tune(self, reps: int = 3) -> str:
+        """Keeps the engine's fastest configuration and returns the report.
+        complex64 batches without dense matrices run on tiles: nothing to tune."""
         buf = C.create_string_buffer(8192)
         N.check(N.lib.plk_batch_tune(self._h, reps, buf, len(buf)))
         return buf.value.decode()
