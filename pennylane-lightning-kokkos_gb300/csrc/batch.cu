@@ -600,7 +600,16 @@ template <class T> static int prepare_run(plk_batch b) {
             PLK_TRY(batch_tiles_create(circs, b->device, b->stream, &b->tiles));
         }
         if (b->tiles) {
-            PLK_TRY(alloc_io(b));
+            const int rc = alloc_io(b);
+            if (rc == PLK_ERR_OUT_OF_MEMORY) { // the engine needs less
+                cudaGetLastError();
+                set_error(std::string());
+                free_device(b);
+            } else {
+                PLK_TRY(rc);
+            }
+        }
+        if (b->tiles) {
             PLK_CUDA(cudaStreamSynchronize(b->stream));
             b->compiled = true;
         } else {

@@ -20,7 +20,8 @@ struct BatchCircuit {
 
 struct BatchTiles; // compiled circuits, their device buffers and launch lists
 
-// nullptr (and PLK_OK) when an op is not of this path (dense matrices)
+// nullptr (and PLK_OK) when an op is not of this path (dense matrices) or the
+// device has no room for the states and programs
 int batch_tiles_create(const std::vector<BatchCircuit> &circs, int device, cudaStream_t st, BatchTiles **out);
 void batch_tiles_destroy(BatchTiles *t);
 // Queues one evaluation: parameters and results on the device; no allocation,
