@@ -496,60 +496,7 @@ __global__ void __launch_bounds__(kThreads, Ctas<A>::apply) k_pauli_apply_tile(c
 }
 
 // --------------------------------------------------------------- host side --
-struct Pass {
-    uint32_t bits = 0;       // state bits of the tile
-    std::vector<int> groups; // indices of the groups inside
-};
-
-int popc(uint64_t x) { return __builtin_popcountll(x); }
-
-// Tiles that cover the groups' X patterns: each pass starts from the widest
-// pattern left, adds patterns that need the fewest more bits, and takes every
-// group that lies inside.
-void choose_passes(int nq, int T, int low, const std::vector<PauliGroup> &groups, std::vector<Pass> &passes,
-                   std::vector<PauliGroup> &rest) {
-    const uint64_t lowmask = (1ull << low) - 1;
-    std::vector<char> done(groups.size(), 0);
-    std::vector<int> order(groups.size());
-    for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-        return popc(groups[a].x & ~lowmask) > popc(groups[b].x & ~lowmask);
-    });
-    for (int seed : order) {
-        if (done[seed]) continue;
-        uint64_t bits = lowmask;
-        Pass p;
-        if (T < nq && popc(bits | groups[seed].x) > T) {
-            done[seed] = 1;
-            rest.push_back(groups[seed]);
-            continue;
-        }
-        bits |= groups[seed].x;
-        for (;;) {
-            int best = -1, cost = 0;
-            for (int i : order) {
-                if (done[i] || (groups[i].x & ~bits) == 0) continue;
-                const int c = popc(bits | groups[i].x);
-                if (c <= T && (best < 0 || c < cost)) {
-                    best = i;
-                    cost = c;
-                }
-            }
-            if (best < 0) break;
-            bits |= groups[best].x;
-        }
-        for (int b = 0; b < nq && popc(bits) < T; b++) bits |= 1ull << b;
-        p.bits = (uint32_t)bits;
-        for (size_t i = 0; i < groups.size(); i++)
-            if (!done[i] && (groups[i].x & ~bits) == 0) {
-                done[i] = 1;
-                p.groups.push_back((int)i);
-            }
-        // one group alone: a plain pass reads the state as often
-        if (p.groups.size() == 1 && T < nq) rest.push_back(groups[p.groups[0]]);
-        else passes.push_back(std::move(p));
-    }
-}
+using Pass = PauliTilePass;
 
 struct Plan {
     std::vector<Pass> passes;
@@ -582,45 +529,6 @@ uint32_t choose_register_bits(const Pass &p, int nq, int T, int low, const std::
     return reg;
 }
 
-// Application: which passes are worth it.  A tile pass reads the state and updates
-// the output for its words; the plain kernel does that once for 32 patterns and
-// gathers each pattern's source.  Costs per tile pass, per word in it, per plain
-// pass and per word in that are times at 24 qubits in us: 40 words of weight 8
-// complex64, some four to a tile pass, 989 on tiles and 605 in plain passes; 40 words
-// of weight 4 450 and 596; complex128 1915 and 2406, 1190 and 2356.
-void keep_worthwhile(bool c64, const std::vector<PauliGroup> &groups, std::vector<Pass> &passes,
-                     std::vector<PauliGroup> &rest) {
-    struct Cost {
-        double pass, word, plain, plain_word;
-    };
-    const Cost c = c64 ? Cost{52, 6.5, 30, 14.5} : Cost{115, 22, 100, 57};
-    auto words = [&](const Pass &p) {
-        int n = 0;
-        for (int gi : p.groups) n += groups[gi].count;
-        return n;
-    };
-    std::stable_sort(passes.begin(), passes.end(), [&](const Pass &x, const Pass &y) { return words(x) > words(y); });
-    // the passes with most words on tiles, the others plain: the cheapest split
-    size_t best = passes.size(), left = rest.size();
-    double least = 0.0, plain = 0.0, on_tiles = 0.0;
-    for (const Pass &p : passes) on_tiles += c.pass + c.word * words(p);
-    for (size_t k = passes.size() + 1; k-- > 0;) {
-        if (k < passes.size()) {
-            on_tiles -= c.pass + c.word * words(passes[k]);
-            plain += c.plain_word * words(passes[k]);
-            left += passes[k].groups.size();
-        }
-        const double cost = on_tiles + plain + c.plain * (double)((left + 31) / 32);
-        if (k == passes.size() || cost < least) {
-            least = cost;
-            best = k;
-        }
-    }
-    for (size_t k = best; k < passes.size(); k++)
-        for (int gi : passes[k].groups) rest.push_back(groups[gi]);
-    passes.resize(best);
-}
-
 // expval: Hermitian form, each pair once
 void make_plan(int nq, int dtype, const std::vector<PauliGroup> &groups, const std::vector<PauliTerm> &terms,
                bool expval, Plan &pl, std::vector<PauliGroup> &rest) {
@@ -629,7 +537,7 @@ void make_plan(int nq, int dtype, const std::vector<PauliGroup> &groups, const s
     const int low = std::min(c64 ? 3 : 2, T);
     const int least = expval ? (c64 ? kManyExpvalC64 : kManyExpvalC128) : (c64 ? kManyApplyC64 : kManyApplyC128);
     choose_passes(nq, T, low, groups, pl.passes, rest);
-    if (!expval) keep_worthwhile(c64, groups, pl.passes, rest);
+    if (!expval) keep_worthwhile(ApplyCost(c64, nq), groups, pl.passes, rest);
     for (const Pass &p : pl.passes) {
         PauliArgs a;
         std::memset((void *)&a, 0, sizeof(a));
@@ -666,7 +574,7 @@ void make_plan(int nq, int dtype, const std::vector<PauliGroup> &groups, const s
             for (int odd = 0; odd < 2; odd++) { // c i^ny is real for an even number of Y, imaginary for an odd one
                 std::vector<const PauliTerm *> words;
                 for (int k = 0; k < g.count; k++)
-                    if ((popc(g.x & terms[g.first + k].z) & 1) == odd) words.push_back(&terms[g.first + k]);
+                    if ((pauli_popc(g.x & terms[g.first + k].z) & 1) == odd) words.push_back(&terms[g.first + k]);
                 if (words.empty()) continue;
                 const bool many = (int)words.size() >= least || (expval && !g.x);
                 // In the expectation value a pair counts twice, and the sign is that of m; applied to m it is that of m ^ x.
@@ -790,12 +698,10 @@ int pauli_tile_expval(plk_state s, const std::vector<PauliGroup> &groups, const 
 int pauli_tile_apply(plk_state out, plk_state in, const std::vector<PauliGroup> &groups,
                      const std::vector<PauliTerm> &terms, std::vector<PauliGroup> &rest, bool &accumulate) {
     accumulate = false;
-    // a tile pass reads the state and updates the output; a plain pass gathers
-    // 32 patterns from the second-level cache or memory
-    // (on small states a launch costs more than its words: 40 words of weight 8, us on
-    // tiles / plain, 13 qubits complex64 49 / 40 and complex128 67 / 73, 16 qubits
-    // 44 / 40 and 85 / 76)
-    if (out->nq < 18 || out->nq > 32 || groups.size() < 2 || !tiles_allowed(out->dtype)) {
+    // below 18 qubits the plain kernel was ahead wherever it was measured (40 words of
+    // weight 8, us on tiles / plain: 13 qubits complex64 49 / 40, 16 qubits 44 / 40)
+    if (out->nq < 18 || out->nq > 32 || groups.size() < 2 || !tiles_allowed(out->dtype) ||
+        !ApplyCost(out->dtype == PLK_C64, out->nq).worth_a_look(groups)) {
         rest = groups;
         return PLK_OK;
     }

@@ -10,22 +10,18 @@
 
 #include <vector>
 
+#include "pauli_plan.hpp"
 #include "plk_internal.cuh"
 
 namespace plk {
 
 // A Pauli word P acts as P|k> = i^ny (-1)^popcount(k & z) |k ^ x>, with x the
 // X/Y positions, z the Y/Z positions, ny the number of Y letters.  Terms that
-// share x form one group.
+// share x form one group (pauli_plan.hpp).
 struct PauliTerm {
     uint64_t z;
     double cr, ci;           // c_j * i^ny
     float crh, crl, cih, cil; // the same, split for the FP32-pipe accumulation
-};
-
-struct PauliGroup {
-    uint64_t x;
-    int first, count;
 };
 
 // The groups that tile passes take; the others (too wide for a tile, alone in
