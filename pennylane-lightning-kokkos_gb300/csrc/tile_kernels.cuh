@@ -791,6 +791,9 @@ __device__ __forceinline__ void run_tile(const Pass &ps, const Buffers &bf, int 
             }
         }
         if (r + 1 < nrounds) {
+            // a tile of fewer threads than a warp: lanes that work alike share their
+            // slots, and all have to have read them before one writes
+            if (T < R + 5) __syncwarp();
 #pragma unroll
             for (int j = 0; j < NA; j++) {
                 A::st(L + slot(j), v[j]);
