@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "gate_ops.cuh"
+#include "sweep_cost.hpp"
 #include "tile_launch.cuh"
 
 namespace plk {
@@ -221,9 +222,9 @@ int apply_ops(plk_state s, const plk_op *ops, int nops, bool &handled) {
 
 // The backward program of a tape; ok stays false when an op is not of this path.
 static int compile_backward(plk_state lam, const plk_op *ops, int nops, const int64_t *tp, int ntp, TileProgram &P,
-                            int &swept, bool &ok) {
+                            std::vector<SweptOp> &swept, bool &ok) {
     ok = false;
-    swept = 0;
+    swept.clear();
     int num_param_ops = 0;
     for (int i = 0; i < nops; i++)
         if (ops[i].num_params > 0) num_param_ops++;
@@ -244,7 +245,7 @@ static int compile_backward(plk_state lam, const plk_op *ops, int nops, const in
                 return PLK_OK;
             invert(L.v);
             c.add(L.v);
-            swept++;
+            swept.push_back({op.gate, trainable});
         } else if (trainable) {
             return PLK_OK;
         }
@@ -255,26 +256,19 @@ static int compile_backward(plk_state lam, const plk_op *ops, int nops, const in
     return PLK_OK;
 }
 
-// 4 state moves per pass and observable, against 2 (1 + nobs) per op for the
-// op-at-a-time kernel that carries every H lambda along.  Adjoint Jacobians of
-// two-term observables, complex128, us in passes / op by op: 12 qubits, 6 ops, 2
-// observables 168 / 376, 8 observables 377 / 684; 20 qubits 6 ops 257 / 450 and
-// 674 / 998, 100 ops 664 / 2681 and 1953 / 8074.
-static bool worth_it(const TileProgram &P, int nobs, int swept) {
-    return nobs == 1 || 4.0 * nobs * P.passes.size() <= 2.0 * (1.0 + nobs) * swept;
-}
-
 // Backward sweeps of all observables; lam is the working copy of the forward
-// state (overwritten).
+// state (overwritten).  plain: the tape is of this path, but cheaper op by op.
 int adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops, const int64_t *tp, int ntp,
-            double *jac, bool &handled) {
-    handled = false;
+            double *jac, bool &handled, bool &plain) {
+    handled = plain = false;
     if (!usable(lam) || ntp <= 0 || nobs < 1) return PLK_OK;
     TileProgram P;
-    int swept = 0;
+    std::vector<SweptOp> swept;
     bool ok = false;
     PLK_TRY(compile_backward(lam, ops, nops, tp, ntp, P, swept, ok));
-    if (!ok || !worth_it(P, nobs, swept)) return PLK_OK;
+    if (!ok) return PLK_OK;
+    plain = !tiles_pay(nobs, lam->dtype == PLK_C64, P, swept);
+    if (plain) return PLK_OK;
     // several sweeps start from lambda: each works on its own copy
     const size_t bytes = lam->length * amp_bytes(lam->dtype);
     int group = std::min(nobs, kMaxSweeps);
@@ -314,10 +308,10 @@ static int adjoint_words(plk_state lam, const std::vector<Word> &words, const pl
     const int nobs = (int)words.size();
     if (!usable(lam) || ntp <= 0 || nobs < 1) return PLK_OK;
     TileProgram P;
-    int swept = 0;
+    std::vector<SweptOp> swept;
     bool ok = false;
     PLK_TRY(compile_backward(lam, ops, nops, tp, ntp, P, swept, ok));
-    if (!ok || !worth_it(P, nobs, swept)) return PLK_OK;
+    if (!ok || !tiles_pay(nobs, lam->dtype == PLK_C64, P, swept)) return PLK_OK;
     DeviceCtx *d = nullptr;
     PLK_TRY(device_ctx(lam->device, &d));
     const size_t bytes = std::max<size_t>(256, lam->length * amp_bytes(lam->dtype));

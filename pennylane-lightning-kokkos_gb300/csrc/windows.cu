@@ -284,7 +284,7 @@ bool window_path_enabled() { return g_window_path.load() != 0; }
 namespace tile { // tile_sweep.cu: everything but dense matrices
 int apply_ops(plk_state s, const plk_op *ops, int nops, bool &handled);
 int adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops, const int64_t *tp, int ntp,
-            double *jac, bool &handled);
+            double *jac, bool &handled, bool &plain);
 } // namespace tile
 
 // Forward: the whole op list through tiles, or through windows.
@@ -399,8 +399,11 @@ static int window_adjoint_concurrent(plk_state lam, plk_state *hls, int nobs, co
 // `lam` is the working copy of the forward state (overwritten).
 int window_adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops, const int64_t *tp, int ntp,
                    double *jac, bool &handled) {
-    PLK_TRY(tile::adjoint(lam, hls, nobs, ops, nops, tp, ntp, jac, handled));
-    if (handled) return PLK_OK;
+    // where tiles lose to the gates' own kernels, windows do so by more (22 qubits
+    // complex128, 60 IsingXY, 16 observables: 30 ms on tiles, 31 op by op, 111 in windows)
+    bool plain = false;
+    PLK_TRY(tile::adjoint(lam, hls, nobs, ops, nops, tp, ntp, jac, handled, plain));
+    if (handled || plain) return PLK_OK;
     if (!window_path_enabled() || (lam->dtype != PLK_C64 && !c128_use_df()) || lam->nq < 6 || lam->nq > 32 ||
         ntp <= 0)
         return PLK_OK;
