@@ -563,7 +563,7 @@ struct LaunchItem {
 
 struct BatchTiles {
     int device = 0;
-    std::vector<void *> buffers;
+    void *block = nullptr; // what the pointers below point into
     SymEval *evals = nullptr;
     SymRun *runs = nullptr;
     SymGate *gates = nullptr;
@@ -587,8 +587,7 @@ struct BatchTiles {
     int nevals = 0, nruns = 0, ntables = 0, npatches = 0, nslots = 0, ncirc = 0;
     std::vector<LaunchItem> launches;
     ~BatchTiles() {
-        for (void *p : buffers)
-            if (p) cudaFree(p);
+        if (block) cudaFree(block);
     }
 };
 
@@ -598,21 +597,52 @@ int batch_tiles_launches(const BatchTiles *t) { return (int)t->launches.size() +
 
 namespace {
 
-template <class V> int upload(BatchTiles *t, V *&dst, const std::vector<V> &src, cudaStream_t st) {
-    void *p = nullptr;
-    PLK_CUDA(cudaMalloc(&p, std::max<size_t>(src.size(), 1) * sizeof(V)));
-    t->buffers.push_back(p);
-    dst = static_cast<V *>(p);
-    if (!src.empty()) PLK_CUDA(cudaMemcpyAsync(p, src.data(), src.size() * sizeof(V), cudaMemcpyHostToDevice, st));
-    return PLK_OK;
-}
-template <class V> int reserve(BatchTiles *t, V *&dst, size_t n) {
-    void *p = nullptr;
-    PLK_CUDA(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(V)));
-    t->buffers.push_back(p);
-    dst = static_cast<V *>(p);
-    return PLK_OK;
-}
+// One allocation for everything a batch has on the device, and one copy for what is
+// small: 22 allocations and 16 copies took 40 us more of the 0.6-0.8 ms of a small
+// batch's first run, and as much of its 0.3 ms of destruction.
+class Block {
+  public:
+    template <class V> void upload(V *&dst, const std::vector<V> &src) {
+        parts_.push_back({reinterpret_cast<void **>(&dst), src.data(), src.size() * sizeof(V), 0});
+    }
+    template <class V> void reserve(V *&dst, size_t n) {
+        parts_.push_back({reinterpret_cast<void **>(&dst), nullptr, n * sizeof(V), 0});
+    }
+    // allocates, points every dst into the block and queues the copies (the sources
+    // stay until the stream is waited for)
+    int commit(void *&block, cudaStream_t st) {
+        constexpr size_t kSmall = 65536;
+        auto place = [&](bool small, size_t at) {
+            for (Part &p : parts_)
+                if ((p.src && p.bytes <= kSmall) == small) {
+                    p.at = at;
+                    at += (std::max<size_t>(p.bytes, 1) + 255) & ~(size_t)255;
+                }
+            return at;
+        };
+        const size_t front = place(true, 0), total = place(false, front);
+        PLK_CUDA(cudaMalloc(&block, std::max<size_t>(total, 256)));
+        host_.assign(front, 0);
+        for (Part &p : parts_) {
+            unsigned char *dst = static_cast<unsigned char *>(block) + p.at;
+            *p.dst = dst;
+            if (!p.src || !p.bytes) continue;
+            if (p.bytes <= kSmall) std::memcpy(host_.data() + p.at, p.src, p.bytes);
+            else PLK_CUDA(cudaMemcpyAsync(dst, p.src, p.bytes, cudaMemcpyHostToDevice, st));
+        }
+        if (front) PLK_CUDA(cudaMemcpyAsync(block, host_.data(), front, cudaMemcpyHostToDevice, st));
+        return PLK_OK;
+    }
+
+  private:
+    struct Part {
+        void **dst;
+        const void *src;
+        size_t bytes, at;
+    };
+    std::vector<Part> parts_;
+    std::vector<unsigned char> host_;
+};
 
 int build(BatchTiles *t, const std::vector<BatchCircuit> &circs, const BasisTable &bt, std::vector<Compiled> &cc,
           cudaStream_t st) {
@@ -801,28 +831,30 @@ int build(BatchTiles *t, const std::vector<BatchCircuit> &circs, const BasisTabl
     t->npatches = (int)patches.size();
     t->nslots = nslots;
     t->ncirc = (int)circs.size();
-    PLK_TRY(upload(t, t->evals, evals, st));
-    PLK_TRY(upload(t, t->runs, runs, st));
-    PLK_TRY(upload(t, t->gates, gates, st));
-    PLK_TRY(upload(t, t->tables, tables, st));
-    PLK_TRY(upload(t, t->factors, factors, st));
-    PLK_TRY(upload(t, t->patches, patches, st));
-    PLK_TRY(upload(t, t->pass_at, pass_at, st));
-    PLK_TRY(upload(t, t->basis, bt.v, st));
-    PLK_TRY(upload(t, t->blobs, blobs, st));
-    PLK_TRY(upload(t, t->jobs, jobs, st));
-    PLK_TRY(upload(t, t->ctas, ctas, st));
-    PLK_TRY(upload(t, t->hctas, hctas, st));
-    PLK_TRY(upload(t, t->terms, terms, st));
-    PLK_TRY(upload(t, t->jfirst, first, st));
-    PLK_TRY(upload(t, t->jterms, jterms, st));
-    PLK_TRY(upload(t, t->ev_range, ev_range, st));
-    PLK_TRY(reserve(t, t->pool, npool));
-    PLK_TRY(reserve(t, t->rot, runs.size()));
-    PLK_TRY(reserve(t, t->refs, nrefs));
-    PLK_TRY(reserve(t, t->states, most));
-    PLK_TRY(reserve(t, t->part, npart));
-    PLK_TRY(reserve(t, t->ev_part, hctas.size()));
+    Block b;
+    b.upload(t->evals, evals);
+    b.upload(t->runs, runs);
+    b.upload(t->gates, gates);
+    b.upload(t->tables, tables);
+    b.upload(t->factors, factors);
+    b.upload(t->patches, patches);
+    b.upload(t->pass_at, pass_at);
+    b.upload(t->basis, bt.v);
+    b.upload(t->blobs, blobs);
+    b.upload(t->jobs, jobs);
+    b.upload(t->ctas, ctas);
+    b.upload(t->hctas, hctas);
+    b.upload(t->terms, terms);
+    b.upload(t->jfirst, first);
+    b.upload(t->jterms, jterms);
+    b.upload(t->ev_range, ev_range);
+    b.reserve(t->pool, npool);
+    b.reserve(t->rot, runs.size());
+    b.reserve(t->refs, nrefs);
+    b.reserve(t->states, most);
+    b.reserve(t->part, npart);
+    b.reserve(t->ev_part, hctas.size());
+    PLK_TRY(b.commit(t->block, st));
     PLK_CUDA(cudaFuncSetAttribute(k_batch_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem_bytes(8, false, kBT, kBBlob, 0, kBThreads)));
     PLK_CUDA(cudaFuncSetAttribute(k_batch_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -857,7 +889,13 @@ int batch_tiles_create(const std::vector<BatchCircuit> &circs, int device, cudaS
             }
         }
     };
-    const unsigned n = std::min<size_t>({std::max(1u, std::thread::hardware_concurrency()), 16, (circs.size() + 7) / 8});
+    // by ops, not by circuits: an op takes some 2 us to compile, both ways, a thread
+    // 20-30 us to start (16 circuits of 12 qubits and 100 layers, first run: 2 threads
+    // 32.5 ms, 16 threads 14.2; two circuits of 70 ops 0.58 ms with one, 0.65 with two)
+    size_t nops = 0;
+    for (const BatchCircuit &c : circs) nops += c.ops->size();
+    const unsigned n =
+        std::min<size_t>({std::max(1u, std::thread::hardware_concurrency()), 16, circs.size(), 1 + nops / 1024});
     std::vector<std::thread> pool;
     for (unsigned k = 1; k < n; k++) {
         try {
