@@ -48,7 +48,8 @@ struct Args {
     uint32_t prog_bytes;
     int T, nacc, ntiles;
     int nacc_all;      // accumulators of the whole program
-    int in_df, out_df; // complex128: buffers hold double-float pairs on entry / exit
+    int in_df, out_df; // complex128: buffers hold doubles (0) or double-float pairs (1) on entry / exit, or
+                       // doubles that a program of index maps alone moves as they are (2)
     int drop;          // the states on exit are not wanted
     double *part;      // [sweep][accumulator][gridDim.x]
     // when set, H lambda of sweep y starts as the Pauli word i^ny (-1)^popcount(k & z) |k ^ x> on lam_src[y]
@@ -561,11 +562,11 @@ __device__ __forceinline__ void store_amp(void *p, uint32_t i, int, f2x v) {
 // low part unnormalised, it collects rounding errors and is itself rounded at
 // their size (state errors over a list of gates: 1.9e-13 without, 6e-14 with).
 __device__ __forceinline__ void store_amp(void *p, uint32_t i, int df, AmpC128::V v) {
-    if (df) {
+    if (df == 1) {
         const f2x s = f2x_add(v.h, v.l);
         v.l = f2x_sub(v.l, f2x_sub(s, v.h));
         v.h = s;
-    } else {
+    } else if (df == 0) {
         const double re = df_join(f2x_lo(v.h), f2x_lo(v.l)), im = df_join(f2x_hi(v.h), f2x_hi(v.l));
         v = {(f2x)__double_as_longlong(re), (f2x)__double_as_longlong(im)};
     }
@@ -623,7 +624,7 @@ struct RoundHead {
 struct Buffers {
     const void *lam_src;
     void *lam, *hl;
-    int in_df, out_df; // complex128: double-float pairs on entry / exit
+    int in_df, out_df; // complex128: what the buffers hold on entry / exit, as in Args
     bool from_zero;    // the state is |0...0> on entry, lam_src is not read
     bool drop;         // the states on exit are not written: a backward sweep's last pass on buffers of its own
                        // (Jacobian of 20 observables on 20 qubits complex128 30.21 -> 30.06 ms)

@@ -41,3 +41,35 @@ def test_reruns(nq, dtype):
     np.testing.assert_allclose(jac, O.adjoint_jacobian(psi, obs, ops, trainable), atol=JTOL[dtype], rtol=0)
     for _ in range(5):
         np.testing.assert_array_equal(gpu_adjoint(psi, obs, ops, trainable, dtype), jac)
+
+
+@pytest.mark.parametrize("nq", [4, 5, 8, 11, 13, 15])
+def test_index_maps_move_doubles_exactly(nq):
+    """CNOT, X and SWAP alone, one pass or several: every bit of a double arrives, also
+    of what double-float cannot hold."""
+    rng = np.random.default_rng(nq)
+    ops = []
+    for _ in range(50 if nq < 13 else 80):
+        name = str(rng.choice(["CNOT", "PauliX", "SWAP"]))
+        ops.append((name, [int(w) for w in rng.choice(nq, 1 if name == "PauliX" else 2, replace=False)], False, []))
+    psi = rand_state(nq, rng)
+    psi[: 4] = [1e-200 + 3e-310j, -1e200j, complex(np.inf, 0.1), complex(np.nan, -0.0)]
+    ref = psi.copy()
+    for name, w, _, _ in ops: # by index, so that no arithmetic meets inf and nan
+        i = np.arange(1 << nq)
+        bit = [i >> (nq - 1 - x) & 1 for x in w]
+        if name == "PauliX":
+            src = i ^ (1 << (nq - 1 - w[0]))
+        elif name == "CNOT":
+            src = i ^ (bit[0] << (nq - 1 - w[1]))
+        else:
+            d = bit[0] ^ bit[1]
+            src = i ^ (d << (nq - 1 - w[0])) ^ (d << (nq - 1 - w[1]))
+        ref = ref[src]
+    s = State.from_array(psi, N.PLK_C128)
+    arr, keep = make_ops(ops)
+    N.check(N.lib.plk_apply_ops(s.h, arr, len(ops)))
+    got = s.get()
+    s.close()
+    del keep
+    np.testing.assert_array_equal(got.view(np.uint64), ref.view(np.uint64))
