@@ -590,6 +590,7 @@ class Compiler {
             if (indeg_[i] == 0) ready.push_back(i);
         deg_.assign(units_.size(), 0);
         in_.assign(units_.size(), 0);
+        used_.assign(groups_.size(), 0);
         pend_ = 1;
         last_table_ = Table{};
         size_t done = 0;
@@ -621,11 +622,16 @@ class Compiler {
                 sel.resize(sel.size() * 3 / 4);
             }
             if (pass.blob.size() > o_.max_blob) return false;
-            for (int i : sel) {
-                ready.erase(std::find(ready.begin(), ready.end(), i));
-                for (int s : succ_[i])
-                    if (--indeg_[s] == 0) insert_sorted(ready, s);
-            }
+            for (int i : sel) in_[i] = 1;
+            ready.erase(std::remove_if(ready.begin(), ready.end(), [&](int i) { return in_[i] != 0; }), ready.end());
+            for (int i : sel)
+                for (int k = inc0_[i]; k < inc0_[i + 1]; k++) {
+                    const Group &g = groups_[inc_[k].group];
+                    if (--groups_[inc_[k].group].left > 0 || g.next < 0) continue;
+                    for (int q = groups_[g.next].head; q >= 0; q = inc_[q].next)
+                        if (--indeg_[inc_[q].unit] == 0 && !in_[inc_[q].unit]) insert_sorted(ready, inc_[q].unit);
+                }
+            for (int i : sel) in_[i] = 0;
             done += sel.size();
             P.nacc += nacc;
             P.jac.insert(P.jac.end(), jac.begin(), jac.end());
@@ -655,10 +661,26 @@ class Compiler {
     std::vector<Prim> prims_;
     std::vector<int> last_; // last primitive touching each bit
     std::vector<Unit> units_;
-    std::vector<std::vector<int>> succ_;
-    std::vector<int> indeg_;
-    std::vector<int> deg_;  // scratch: in-degrees inside a selection
-    std::vector<char> in_;  // scratch: members of a selection
+    // The dependency graph.  The units on a state bit form groups that commute there
+    // (all D, all F, or one unit); a unit waits, on each of its bits, for the whole group
+    // before its own.  Groups, not pairs of units: lists of thousands of commuting
+    // gates have as many groups as bits.
+    struct Group {
+        Access a = AC_N;
+        int prev = -1, next = -1; // groups of the same bit
+        int left = 0;             // units not done
+        int head = -1, tail = -1; // first and last incidence
+    };
+    struct Incidence { // a unit in a group
+        int unit, group, next;
+    };
+    std::vector<Group> groups_;
+    std::vector<Incidence> inc_;
+    std::vector<int> inc0_;  // a unit's first incidence (and one past the last unit)
+    std::vector<int> indeg_; // groups that a unit waits for
+    std::vector<int> deg_;   // scratch: of these, inside a selection
+    std::vector<int> used_;  // scratch: selected units of a group
+    std::vector<char> in_;   // scratch: members of a selection
     // complex128: the state is pend_ times what the sweep holds
     double pend_ = 1;
     struct Table { // the last phase table: pass, first entry, Jacobian terms before it
@@ -1036,45 +1058,46 @@ class Compiler {
 
     void make_graph() {
         const int n = (int)units_.size();
-        succ_.assign(n, {});
+        groups_.clear();
+        inc_.clear();
+        inc0_.assign(1, 0);
         indeg_.assign(n, 0);
-        struct Group {
-            Access a = AC_N;
-            std::vector<int> cur, prev;
-        };
-        std::vector<Group> g(nq_);
-        std::vector<int> mark(n, -1);
-        for (int i = 0; i < n; i++)
+        std::vector<int> last(nq_, -1); // present group of a bit
+        for (int i = 0; i < n; i++) {
             for (uint32_t m = units_[i].bits; m; m &= m - 1) {
-                const int b = __builtin_ctz(m);
-                Group &q = g[b];
+                const int b = __builtin_ctz(m), before = last[b];
                 const Access a = access(units_[i], b);
-                if (!(a != AC_N && a == q.a && !q.cur.empty())) {
-                    std::swap(q.prev, q.cur);
-                    q.cur.clear();
-                    q.a = a;
+                if (before < 0 || a == AC_N || groups_[before].a != a) {
+                    Group g;
+                    g.a = a;
+                    g.prev = before;
+                    last[b] = (int)groups_.size();
+                    if (before >= 0) groups_[before].next = last[b];
+                    groups_.push_back(g);
                 }
-                for (int j : q.prev)
-                    if (mark[j] != i) {
-                        mark[j] = i;
-                        succ_[j].push_back(i);
-                        indeg_[i]++;
-                    }
-                q.cur.push_back(i);
+                Group &g = groups_[last[b]];
+                (g.tail < 0 ? g.head : inc_[g.tail].next) = (int)inc_.size();
+                g.tail = (int)inc_.size();
+                g.left++;
+                if (g.prev >= 0) indeg_[i]++;
+                inc_.push_back({i, last[b], -1});
             }
+            inc0_.push_back((int)inc_.size());
+        }
     }
 
     // the units of the next pass, in an order that respects the graph
     void select(const std::vector<int> &ready0, std::vector<int> &sel, uint32_t &bits) {
-        std::vector<int> ready = ready0, touched;
+        std::vector<int> ready = ready0, touched, touched_groups;
         sel.clear();
         if (T_ >= nq_) bits = nq_ >= 32 ? 0xffffffffu : (1u << nq_) - 1;
         else bits = (1u << o_.low) - 1;
         int acc = 0;
+        size_t from = 0; // those before it do not fit, and will not while `bits` stays as it is
         while (!ready.empty() && (int)sel.size() < kMaxUnits) {
             int pick = -1;
             for (int pass = 0; pass < 2 && pick < 0; pass++)
-                for (size_t r = 0; r < ready.size() && pick < 0; r++) {
+                for (size_t r = pass == 0 ? from : 0; r < ready.size() && pick < 0; r++) {
                     const Unit &u = units_[ready[r]];
                     if (acc + u.ngrad() > kMaxAcc) continue;
                     if (pass == 0 ? (u.need & ~bits) == 0 : popc(bits | u.need) <= T_) pick = (int)r;
@@ -1082,15 +1105,27 @@ class Compiler {
             if (pick < 0) break;
             const int i = ready[pick];
             ready.erase(ready.begin() + pick);
+            from = (units_[i].need & ~bits) ? 0 : (size_t)pick;
             bits |= units_[i].need;
             acc += units_[i].ngrad();
             sel.push_back(i);
-            for (int s : succ_[i]) {
-                if (deg_[s]++ == 0) touched.push_back(s);
-                if (deg_[s] == indeg_[s]) insert_sorted(ready, s);
+            for (int k = inc0_[i]; k < inc0_[i + 1]; k++) {
+                const int gi = inc_[k].group;
+                const Group &g = groups_[gi];
+                if (used_[gi]++ == 0) touched_groups.push_back(gi);
+                if (used_[gi] < g.left || g.next < 0) continue;
+                for (int q = groups_[g.next].head; q >= 0; q = inc_[q].next) {
+                    const int s = inc_[q].unit;
+                    if (deg_[s]++ == 0) touched.push_back(s);
+                    if (deg_[s] < indeg_[s]) continue;
+                    const auto at = std::lower_bound(ready.begin(), ready.end(), s);
+                    from = std::min(from, (size_t)(at - ready.begin()));
+                    ready.insert(at, s);
+                }
             }
         }
         for (int s : touched) deg_[s] = 0;
+        for (int g : touched_groups) used_[g] = 0;
         for (int b = 0; b < nq_ && popc(bits) < T_; b++) bits |= 1u << b; // fill with low bits
     }
 
@@ -1576,20 +1611,33 @@ class Compiler {
         identity(o.col, T_);
         identity(o.out, T_);
         nacc = 0;
-        for (int i : sel) in_[i] = 1;
-        for (int i : sel)
-            for (int s : succ_[i])
-                if (in_[s]) deg_[s]++;
+        for (int i : sel) {
+            in_[i] = 1;
+            for (int k = inc0_[i]; k < inc0_[i + 1]; k++) used_[inc_[k].group]++;
+        }
         std::vector<int> ready;
-        for (int i : sel)
+        for (int i : sel) {
+            for (int k = inc0_[i]; k < inc0_[i + 1]; k++) {
+                const int before = groups_[inc_[k].group].prev;
+                deg_[i] += before >= 0 && used_[before] > 0;
+            }
             if (deg_[i] == 0) insert_sorted(ready, i);
+        }
         size_t left = sel.size();
+        // a group's selected units that are left, counted down from its units not done:
+        // the next group is in the selection only where all of them are
+        for (int i : sel)
+            for (int k = inc0_[i]; k < inc0_[i + 1]; k++) used_[inc_[k].group] = groups_[inc_[k].group].left;
         auto finish = [&](size_t r) {
             const int i = ready[r];
             ready.erase(ready.begin() + r);
             left--;
-            for (int s : succ_[i])
-                if (in_[s] && --deg_[s] == 0) insert_sorted(ready, s);
+            for (int k = inc0_[i]; k < inc0_[i + 1]; k++) {
+                const int gi = inc_[k].group, after = groups_[gi].next;
+                if (--used_[gi] > 0 || after < 0) continue;
+                for (int q = groups_[after].head; q >= 0; q = inc_[q].next)
+                    if (in_[inc_[q].unit] && --deg_[inc_[q].unit] == 0) insert_sorted(ready, inc_[q].unit);
+            }
         };
         bool ok = true;
         std::vector<Step> st;
@@ -1623,7 +1671,11 @@ class Compiler {
             for (int k = T_ - 1; k >= 0 && popc(regs) < R_; k--) regs |= 1u << o.tbits[k];
             ok = !st.empty() && emit_round(o, st, regs, acc0, jac, nacc);
         }
-        for (int i : sel) in_[i] = 0, deg_[i] = 0;
+        for (int i : sel) {
+            in_[i] = 0;
+            deg_[i] = 0;
+            for (int k = inc0_[i]; k < inc0_[i + 1]; k++) used_[inc_[k].group] = 0;
+        }
         if (!ok || nacc > kMaxAcc * 2) return false;
         // the last round writes the state: through the map from its indices to
         // the present ones, or, where its lanes do not cover the lowest state
