@@ -265,8 +265,9 @@ PLK_API int plk_expval_pauliz_noalloc(const void *state, int32_t num_qubits, int
  * over shared-memory tiles of 2^11 to 2^12 amplitudes), or, with dense
  * matrices in the list, as register windows of four bits; complex128 in
  * double-float on the FP32 pipe; with several observables one backward sweep
- * per observable on a copy of lambda, when that moves fewer bytes.  Results
- * agree with the op-at-a-time path to rounding. */
+ * per observable on a copy of lambda, when that is estimated to take less time
+ * than the gates' own kernels.  Lists of CNOT, X and SWAP alone move amplitudes
+ * bit for bit.  Results agree with the op-at-a-time path to rounding. */
 PLK_API int plk_set_window_path(int32_t enable);
 PLK_API int plk_get_window_path(int32_t *enabled);
 
@@ -311,8 +312,8 @@ PLK_API int plk_gate_matrix(int32_t gate, const double *params, int32_t num_para
  * parameters, own Pauli-sum observable) evaluated together: for every circuit
  * the forward pass from |0...0>, <H> and the adjoint gradient d<H>/dtheta of
  * its trainable parameters, in a fixed sequence of launches (replayed as a CUDA
- * graph; complex128 batches and batches with dense matrices in one persistent
- * launch).  Per circuit this is what the reference's device does one tape at
+ * graph; complex128 batches, batches with dense matrices and those whose states
+ * and programs the device has no room for, in one persistent launch).  Per circuit this is what the reference's device does one tape at
  * a time: apply the tape (StateVectorKokkos::applyOperation,
  * StateVectorKokkos.hpp:585-676), the Hamiltonian expectation
  * (ObservablesKokkos.hpp:484-494) and AdjointJacobianKokkos::adjointJacobian

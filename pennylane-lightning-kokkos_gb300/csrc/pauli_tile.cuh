@@ -4,8 +4,8 @@
 // pattern reads it as many times as there are patterns; here a pass holds tiles
 // of 2^T amplitudes in shared memory, the tile's bits chosen so that as many
 // patterns as possible lie inside them, and evaluates all of those words on the
-// tile it has read once.  100 random words of weight 1-4 on 26 wires take about
-// a dozen passes instead of 90.
+// tile it has read once.  100 random words of weight 1-4 on 26 wires, 68 to 80
+// patterns, take 5 or 6 passes.
 #pragma once
 
 #include <vector>

@@ -8,8 +8,8 @@
 //
 // Fitted to Jacobians of 8 and of 60 gates of each kind on random wires, 2-16
 // observables, 10-24 qubits, both precisions, with the path switched on and off:
-// tiles within 5 % (22 and 24 qubits), gates within 8 %, and the dearer way is
-// taken in 37 of 2924, by 24 % at most.  22 qubits complex128, 60 gates, 3
+// tiles 4-6 % rms, gates 7-8 % (22 and 24 qubits), and the dearer way is taken in
+// 37 of 2924, by 24 % at most.  22 qubits complex128, 60 gates, 3
 // observables, ms on tiles / op by op: DoubleExcitation (an eighth of the state
 // each) 5.8 / 2.7, CSWAP 6.3 / 3.0, Toffoli 5.3 / 2.9, RX 1.8 / 9.4, IsingXX 5.2 / 8.9.
 //
