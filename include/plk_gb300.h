@@ -237,7 +237,8 @@ PLK_API int plk_adjoint_jacobian_inplace(plk_state lambda, plk_state *hlambda, i
 
 /* The same Jacobian for observables that are one Pauli word each (observable o:
  * coeffs[o] times the letters offsets[o] .. offsets[o+1]) without the caller
- * forming H lambda: the sweep reads it off lambda, which is not modified.
+ * forming H lambda: the sweep reads it off lambda, which is not modified (or, for
+ * tapes that are cheaper gate by gate, the states are formed inside).
  * PLK_ERR_UNSUPPORTED when the tape or the free memory does not allow it (then
  * form the states and call plk_adjoint_jacobian). */
 PLK_API int plk_adjoint_jacobian_pauli(plk_state lambda, int32_t num_obs, const double *coeffs, const int64_t *offsets,

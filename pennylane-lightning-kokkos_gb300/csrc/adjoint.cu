@@ -209,6 +209,14 @@ int adjoint_checks(plk_state lambda, plk_state *hlambda, int32_t nobs, const plk
     return PLK_OK;
 }
 
+// The sweep gate by gate: every H lambda is carried along, all on work's stream;
+// work and the observables' states are overwritten.
+int adjoint_gates(plk_state work, plk_state *hlambda, int32_t nobs, const plk_op *ops, int32_t nops,
+                  const int64_t *trainable, int32_t ntp, double *jac) {
+    return work->dtype == PLK_C64 ? adjoint_impl<float>(work, hlambda, nobs, ops, nops, trainable, ntp, jac)
+                                  : adjoint_impl<double>(work, hlambda, nobs, ops, nops, trainable, ntp, jac);
+}
+
 } // namespace plk
 
 using namespace plk;
@@ -227,9 +235,7 @@ static int adjoint_run(plk_state work, plk_state *hlambda, int32_t nobs, const p
     }
     bool handled = false;
     if (st == PLK_OK) st = window_adjoint(work, hlambda, nobs, ops, nops, trainable, ntp, jac, handled);
-    if (st == PLK_OK && !handled)
-        st = work->dtype == PLK_C64 ? adjoint_impl<float>(work, hlambda, nobs, ops, nops, trainable, ntp, jac)
-                                    : adjoint_impl<double>(work, hlambda, nobs, ops, nops, trainable, ntp, jac);
+    if (st == PLK_OK && !handled) st = adjoint_gates(work, hlambda, nobs, ops, nops, trainable, ntp, jac);
     const std::string err = st == PLK_OK ? std::string() : last_error();
     for (int o = 0; o < nobs; o++)
         if (old_streams[o]) plk_state_set_stream(hlambda[o], old_streams[o]);

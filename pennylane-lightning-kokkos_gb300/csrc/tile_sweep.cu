@@ -17,6 +17,8 @@
 namespace plk {
 
 bool window_path_enabled();
+int adjoint_gates(plk_state work, plk_state *hlambda, int32_t nobs, const plk_op *ops, int32_t nops,
+                  const int64_t *trainable, int32_t ntp, double *jac);
 int plan_generator(int gate, int nw, GatePlan &p);
 
 namespace tile {
@@ -305,6 +307,33 @@ int adjoint(plk_state lam, plk_state *hls, int nobs, const plk_op *ops, int nops
     return PLK_OK;
 }
 
+// Words whose tape is cheaper gate by gate: their states are formed here, so that
+// the caller does not compile the tape once more to learn the same.
+static int adjoint_word_states(plk_state lam, const std::vector<Word> &words, const plk_op *ops, int nops,
+                               const int64_t *tp, int ntp, double *jac) {
+    std::vector<plk_state> made; // the working copy of lambda, then H lambda of each word
+    int rc = PLK_OK;
+    for (size_t o = 0; o <= words.size() && rc == PLK_OK; o++) {
+        plk_state s = nullptr;
+        rc = plk_state_create(lam->nq, lam->dtype, lam->device, &s);
+        if (rc != PLK_OK) break;
+        made.push_back(s);
+        rc = plk_state_set_stream(s, lam->stream);
+        if (rc == PLK_OK) rc = plk_state_copy(s, lam);
+        for (int b = 0; o > 0 && b < lam->nq && rc == PLK_OK; b++) {
+            const Word &w = words[o - 1];
+            const int gate = (w.x & w.z) >> b & 1 ? PLK_GATE_PAULIY : w.x >> b & 1 ? PLK_GATE_PAULIX : PLK_GATE_PAULIZ;
+            const int64_t wire = lam->nq - 1 - b;
+            if ((w.x | w.z) >> b & 1) rc = plk_apply_gate(s, gate, &wire, 1, 0, nullptr, 0);
+        }
+    }
+    if (rc == PLK_OK) rc = adjoint_gates(made[0], made.data() + 1, (int)words.size(), ops, nops, tp, ntp, jac);
+    const std::string err = rc == PLK_OK ? std::string() : last_error();
+    for (plk_state s : made) plk_state_destroy(s);
+    if (rc != PLK_OK) set_error(err);
+    return rc;
+}
+
 // Observables that are one Pauli word each: H lambda is never stored, the first
 // pass reads it as the permuted, signed lambda (which is not modified).
 static int adjoint_words(plk_state lam, const std::vector<Word> &words, const plk_op *ops, int nops, const int64_t *tp,
@@ -316,20 +345,23 @@ static int adjoint_words(plk_state lam, const std::vector<Word> &words, const pl
     std::vector<SweptOp> swept;
     bool ok = false;
     PLK_TRY(compile_backward(lam, ops, nops, tp, ntp, P, swept, ok));
-    if (!ok || !tiles_pay(nobs, lam->dtype == PLK_C64, P, swept)) return PLK_OK;
+    if (!ok) return PLK_OK;
+    const bool gates = !tiles_pay(nobs, lam->dtype == PLK_C64, P, swept);
     DeviceCtx *d = nullptr;
     PLK_TRY(device_ctx(lam->device, &d));
     const size_t bytes = std::max<size_t>(256, lam->length * amp_bytes(lam->dtype));
     const int group =
         (int)std::min<size_t>(std::min(nobs, kMaxSweeps), std::max<size_t>(1, ((size_t)4 << 30) / (2 * bytes)));
     PoolBuf buf(lam->stream);
-    if (cudaMallocFromPoolAsync(&buf.p, 2 * bytes * group, d->pool, lam->stream) != cudaSuccess) {
+    if (gates) {
+        PLK_TRY(adjoint_word_states(lam, words, ops, nops, tp, ntp, jac));
+    } else if (cudaMallocFromPoolAsync(&buf.p, 2 * bytes * group, d->pool, lam->stream) != cudaSuccess) {
         cudaGetLastError();
         buf.p = nullptr;
         return PLK_OK; // the caller has ways that need less
     }
     handled = true;
-    for (int o0 = 0; o0 < nobs; o0 += group) {
+    for (int o0 = 0; o0 < nobs && !gates; o0 += group) {
         const int n = std::min(group, nobs - o0);
         const void *src[kMaxSweeps];
         void *dst[kMaxSweeps], *h[kMaxSweeps];
